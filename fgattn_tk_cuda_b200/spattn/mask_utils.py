@@ -88,6 +88,16 @@ class CompressedBitMaskCache(BitMaskCache):
         packed, seq_len = self.cache[layer]
         return packedmask_to_indexmask_cuda(packed, seq_len)
 
+    _own_reading = get_mask_from_cache
+
+    def list_reader(self):
+        """What an attention step reads its lists with: get_lists, unless a program has put a get_mask_from_cache of
+        its own in a subclass, in this class or on the object."""
+        read = self.get_mask_from_cache
+        own = getattr(read, "__self__", None) is self and \
+            getattr(read, "__func__", None) is CompressedBitMaskCache._own_reading
+        return self.get_lists if own else read
+
     def get_lists(self, layer):
         """The same lists for the attention operator alone: slots past the counts hold anything."""
         packed, seq_len = self.cache[layer]
@@ -144,13 +154,13 @@ def packedmask_to_indexmask_cuda(packed: torch.Tensor, seq=None, stride=None):
     return indices, num
 
 
-def _packedmask_to_lists(packed: torch.Tensor, seq: int):
+def _packedmask_to_lists(packed: torch.Tensor, seq=None):
     """packedmask_to_indexmask_cuda without the sentinels: the operators read a list up to its count, and the
     slots behind it are most of the bytes (20 of 21 at 5 % of the keys kept)."""
     W = packed.shape[-1] * 8
     indices = torch.empty((*packed.shape[:-1], W), dtype=torch.int32, device=packed.device)
     num = torch.empty(packed.shape[:-1], dtype=torch.int32, device=packed.device)
-    spattn_interface.packedmask_to_lists(indices, num, packed.contiguous(), seq)
+    spattn_interface.packedmask_to_lists(indices, num, packed.contiguous(), W if seq is None else seq)
     return indices, num
 
 

@@ -128,11 +128,9 @@ def bitmaskcached_attn_cuda(query, key, value, current_layer, ditrun, *args, **k
         mask, _, _, out = mask_utils.qk_token_mask_cuda(query, key, kwargs["thresh"], v=value)
         mask_cache.update_cache(current_layer, mask, key.shape[2])
         return out
-    if type(mask_cache) is mask_utils.CompressedBitMaskCache:
-        mask = mask_cache.get_lists(current_layer)
-    else:
-        mask = mask_cache.get_mask_from_cache(current_layer)
-    return _sparse(_out(query), query, key, value, mask[:2])
+    compressed = isinstance(mask_cache, mask_utils.CompressedBitMaskCache)
+    read = mask_cache.list_reader() if compressed else mask_cache.get_mask_from_cache
+    return _sparse(_out(query), query, key, value, read(current_layer)[:2])
 
 
 def attn_2xmask_cuda(query, key, value, current_layer=None, ditrun=None, *args, **kwargs):

@@ -114,3 +114,48 @@ def test_noalloc_wrapper_refuses_k_of_another_length():
         capi.block_index_lists_noalloc(i32, i32, f32, f32, q, k_short, 1e-3)
     with pytest.raises(capi.FgattnError, match="shape of q"):
         capi.block_index_lists_noalloc(i32, i32, f32, f32, q, q, 1e-3, o=q, v=k_short)
+
+
+def _bit_cache(seq_len):
+    from fgattn_tk_cuda_b200.spattn import mask_utils
+    cache = mask_utils.CompressedBitMaskCache([0])
+    cache.cache[0] = (t(B, H, NQB128, 256 // 8, dtype=torch.uint8), seq_len)
+    return cache
+
+
+def _replay(cache):
+    from fgattn_tk_cuda_b200.spattn import sparseattn_functionals as functionals
+    a = good()
+    return functionals.bitmaskcached_attn_cuda(a["q"], a["k"], a["v"], 0, 1, mask_cache=cache, thresh=1e-3)
+
+
+@pytest.mark.parametrize("seq_len", [None, 0, SKV, 256])
+def test_kept_bits_of_any_valid_length(seq_len):
+    """A kept bit mask whose length is None counts in full width, as packedmask_to_indexmask_cuda takes it."""
+    assert _replay(_bit_cache(seq_len)).shape == (B, H, S, D)
+    assert _bit_cache(seq_len).get_lists(0)[0].shape == (B, H, NQB128, 256)
+
+
+def test_replaced_reading_of_a_kept_mask_is_called(monkeypatch):
+    """A program's own get_mask_from_cache is the one that an attention step reads, whether it sits on the object, in a
+    subclass or in place of the class's."""
+    from fgattn_tk_cuda_b200.spattn import mask_utils
+    calls = []
+
+    def own(*layer):
+        calls.append(layer[-1])
+        return good()["ti"], good()["tc"]
+
+    cache = _bit_cache(SKV)
+    cache.get_mask_from_cache = own
+    _replay(cache)
+
+    class Sub(mask_utils.CompressedBitMaskCache):
+        get_mask_from_cache = own
+
+    sub = Sub([0])
+    sub.cache = _bit_cache(SKV).cache
+    _replay(sub)
+    monkeypatch.setattr(mask_utils.CompressedBitMaskCache, "get_mask_from_cache", own)
+    _replay(_bit_cache(SKV))
+    assert calls == [0, 0, 0]
