@@ -22,6 +22,22 @@ __device__ __forceinline__ void online_init(OnlineState& st) {
   st.l = 0.f;
 }
 
+// Multiplies one row of the accumulator (D fp32 columns at o_addr) by alpha.  Nothing may still be adding to it.  Where
+// the query tile has one score buffer, the commit that published its scores covers its previous P*V product too.  With
+// rotating score buffers the scores come while that product may still be running: the caller waits for it first.
+template <int D>
+__device__ __forceinline__ void rescale_accumulator(uint32_t o_addr, float alpha) {
+#pragma unroll
+  for (int cc = 0; cc < D / 32; ++cc) {
+    uint32_t o[32];
+    tmem_ld32(o_addr + cc * 32, o);
+    tmem_ld_wait();
+#pragma unroll
+    for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
+    tmem_st32(o_addr + cc * 32, o);
+  }
+}
+
 // Online softmax over one score tile.
 //   s_addr : TMEM address (lane already folded in) of the 128 fp32 score columns
 //   p_addr : where the 64 packed-bf16 probability columns go (WRITE_P)
@@ -85,17 +101,7 @@ __device__ __forceinline__ void softmax_online_step(uint32_t s_addr, uint32_t p_
     st.l *= alpha;
     if (WRITE_P && !first) {
       quiet();
-      // the accumulator is quiescent: the commit that published this score tile also covers the
-      // previous P*V product of the same query tile
-#pragma unroll
-      for (int cc = 0; cc < D / 32; ++cc) {
-        uint32_t o[32];
-        tmem_ld32(o_addr + cc * 32, o);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-        tmem_st32(o_addr + cc * 32, o);
-      }
+      rescale_accumulator<D>(o_addr, alpha);
     }
   }
   float sum0 = 0.f, sum1 = 0.f;
@@ -185,12 +191,16 @@ __device__ __forceinline__ void quarter_probs(uint32_t (&r)[32], float qmax, flo
 }
 
 // softmax_online_step with P over a whole, unmasked 128-key score tile that is not the first of its item.  The
-// offset in use may lag the running maximum by up to 2^8, so it hardly ever moves: the exponentials start against
-// the offset as it stands, before the tile's maximum is known and while three quarters of the scores are still on
+// offset in use may lag the running maximum by up to 2^8, so on most inputs it hardly ever moves: the exponentials start
+// against the offset as it stands, before the tile's maximum is known and while three quarters of the scores are still on
 // their way from tensor memory.  Where some row of the warp turns out to need a larger offset, nothing has been
-// written yet and softmax_online_step does the tile over; the results are the same bit for bit.  Taken at D = 64,
-// where the softmax bounds a step: (2, 16, 4096, 64) 0.224 -> 0.217 ms.  At D = 128 it is level to 2.5 % slower
-// (32768 x 512 keys 0.374 -> 0.384 ms): there the two products and the hand-offs pace a step.
+// written yet: the scores are loaded again and the probabilities of all quarters taken against the new one.  The results
+// are those of softmax_online_step bit for bit.  Taken at D = 64, where the softmax bounds a step: (2, 16, 4096, 64),
+// i.i.d. normal q and k, 0.224 -> 0.217 ms.  With scores so far apart that the offset moves in most tiles (deviation of
+// q and k 2 / 3 / 6) softmax_online_step alone takes 0.232 / 0.239 / 0.241 ms, this with the rotating score buffers of
+// the dense kernel 0.225 / 0.239 / 0.247 (0.244 / 0.265 / 0.272 when a tile was done over from its maximum on).
+// At D = 128 it is level to 2.5 % slower (32768 x 512 keys 0.374 -> 0.384 ms): there the two products and the hand-offs
+// pace a step.
 template <int D, int POLY = 2, class Quiet = NoWait>
 __device__ __forceinline__ void softmax_steady_step(uint32_t s_addr, uint32_t p_addr, uint32_t o_addr, float c,
                                                     OnlineState& st, float& mx0, float& mx1, Quiet quiet = Quiet()) {
@@ -212,21 +222,35 @@ __device__ __forceinline__ void softmax_steady_step(uint32_t s_addr, uint32_t p_
   mx0 = fmaxf(qm[0], qm[1]);
   mx1 = fmaxf(qm[2], qm[3]);
   const float mx = fmaxf(mx0, mx1);
-  if (__any_sync(0xffffffffu, mx * c > st.m_used + 8.0f)) {
-    softmax_online_step<D, true, POLY>(s_addr, p_addr, o_addr, 64, 64, c, false, st, mx0, mx1, nullptr, quiet);
+  st.m_true = fmaxf(st.m_true, mx);
+  auto finish = [&](float off, int from) {
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      if (w >= from) quarter_probs<POLY>(r[w], qm[w], c, off, sum2);
+      tmem_st16(p_addr + w * 16, *reinterpret_cast<uint32_t(*)[16]>(&r[w][0]));
+    }
+    float sum0, sum1;
+    f2_unpack(sum2, sum0, sum1);
+    st.l += sum0 + sum1;
+    tmem_st_wait();
+  };
+  const float ms = mx * c;
+  const bool grow = ms > st.m_used + 8.0f;
+  if (__any_sync(0xffffffffu, grow)) {
+    const float alpha = grow ? ex2(st.m_used - ms) : 1.0f;
+    if (grow) st.m_used = ms;
+    st.l *= alpha;
+    quiet();
+    rescale_accumulator<D>(o_addr, alpha);
+#pragma unroll
+    for (int w = 0; w < 4; ++w) tmem_ld32(s_addr + w * 32, r[w]);
+#pragma unroll
+    for (int w = 0; w < 4; ++w) tmem_ld_wait_for(r[w]);
+    sum2 = f2_pack(0.f, 0.f);
+    finish(-st.m_used, 0);
     return;
   }
-  st.m_true = fmaxf(st.m_true, mx);
-  tmem_st16(p_addr, *reinterpret_cast<uint32_t(*)[16]>(&r[0][0]));
-#pragma unroll
-  for (int w = 1; w < 4; ++w) {
-    quarter_probs<POLY>(r[w], qm[w], c, neg_m, sum2);
-    tmem_st16(p_addr + w * 16, *reinterpret_cast<uint32_t(*)[16]>(&r[w][0]));
-  }
-  float sum0, sum1;
-  f2_unpack(sum2, sum0, sum1);
-  st.l += sum0 + sum1;
-  tmem_st_wait();
+  finish(neg_m, 1);
 }
 
 // Write one row of the fp32 accumulator (D columns at o_addr) as bf16, scaled by `inv`.

@@ -1,5 +1,7 @@
 """GPU parity of the dense family (full_attn, fullattn_maxq_denom, maxq_denom) through the C ABI
 against the golden fixtures and the CPU oracle."""
+import math
+
 import numpy as np
 import pytest
 import torch
@@ -178,9 +180,8 @@ def test_output_rows_at_the_edges(S, K, D):
 
 @pytest.mark.parametrize("jump", [0, 200, 383, 640, 1000])
 def test_offset_moves_inside_any_step(jump):
-    """At D = 64 a step computes its exponentials before it knows the tile's maximum and does the tile over when the
-    offset has to move: one key per run of rows that towers over all before it, in the first tile, at the edges of
-    later ones, in every 32-column quarter position, and in a ragged last tile."""
+    """One key per run of rows that towers over all before it, in the first tile, in later ones and in a ragged last
+    one, with 1024 keys and more (test_offset_moves_in_every_quarter goes through the quarters and both query tiles)."""
     from oracle import fgattn_oracle as orc
     capi = _capi()
     B, H, S, K, D = 1, 2, 256, 1100, 64
@@ -199,3 +200,59 @@ def test_offset_moves_inside_any_step(jump):
         _close(o, orc.full_attn(q, k, v, kv_seq_len=kv))
         rm, rl = orc.maxq_denom(q, k, kv_seq_len=kv)
         _check_ml(m, l, rm[:, :, 0, :S], rl[:, :, 0, :S], S)
+
+
+def _moves(q, k):
+    """Where the offset moves after the first key tile: (head, row, tile, column) by the 2^8 rule, scores in fp32."""
+    c = math.log2(math.e) / math.sqrt(q.shape[-1])
+    s = torch.einsum("hqd,hkd->hqk", q[0].float(), k[0].float()) * c
+    found = []
+    for tile in range(0, (s.shape[-1] + 127) // 128):
+        top, col = s[:, :, 128 * tile:128 * tile + 128].max(-1)
+        if tile == 0:
+            used = top.clone()
+            continue
+        grow = top > used + 8.0
+        for h, r in grow.nonzero().tolist():
+            found.append((h, r, tile, int(col[h, r])))
+        used = torch.where(grow, top, used)
+    return found
+
+
+@pytest.mark.parametrize("many", [False, True])
+@pytest.mark.parametrize("shift", [0, 1, 2, 3])
+def test_offset_moves_in_every_quarter(shift, many):
+    """At D = 64 (above 1024 keys) a step computes the exponentials of its first quarter before it knows the tile's
+    maximum, and has to go back where the offset moves.  Single rows in every warp of both query tiles meet a key of
+    their own direction, longer each time, in the corner columns of the quarters of consecutive tiles; `many`: a thread
+    block for every SM and a cut item (its two query tiles apart) on top."""
+    from oracle import fgattn_oracle as orc
+    capi = _capi()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B, H, S, K, D = 1, sms + 2 if many else 2, 256, 1250, 64
+    g = torch.Generator().manual_seed(shift)
+    q, k, v = (torch.randn(B, H, n, D, generator=g).to(torch.bfloat16) for n in (S, K, K))
+    cols = [0, 31, 32, 63, 64, 95, 96, 127]
+    for n, row in enumerate([3, 40, 77, 100, 130, 161, 200, 255]):
+        for i in range(4):                               # four moves in a row, from tile 1 or tile 2 on
+            col = 128 * (1 + n % 2 + i) + cols[(n + 2 * i + 2 * shift) % 8]
+            direction = q[:, :, row].float() / q[:, :, row].float().norm(dim=-1, keepdim=True)
+            k[:, :, col] = ((14 + 9 * i) * direction).to(torch.bfloat16)
+    k[:, :, K - 2] = (60 * q[:, :, 9].float() / q[:, :, 9].float().norm(dim=-1, keepdim=True)).to(torch.bfloat16)   # ragged tile
+    moves = _moves(q, k)
+    for h in range(min(H, 4)):
+        here = [m for m in moves if m[0] == h]
+        assert {(r // 128, c // 32) for _, r, _, c in here} == {(t, w) for t in range(2) for w in range(4)}
+        assert {r // 32 for _, r, _, _ in here} == set(range(8))
+        assert all(any((h, r, t, c) in here for c in range(128)) for r, t in ((3, 1), (3, 2), (255, 2), (255, 3), (9, 9)))
+    o = torch.full((B, H, S, D), float("nan"), dtype=torch.bfloat16, device="cuda")
+    m, l = _ml_buffers(B, H, S)
+    capi.fullattn_maxq_denom(o, m, l, q.cuda(), k.cuda(), v.cuda())
+    capi.check()
+    _close(o, orc.full_attn(q, k, v))
+    rm, rl = orc.maxq_denom(q, k)
+    _check_ml(m, l, rm[:, :, 0, :S], rl[:, :, 0, :S], S)
+    o2 = torch.full_like(o, float("nan"))
+    capi.full_attn(o2, q.cuda(), k.cuda(), v.cuda())
+    capi.check()
+    assert torch.equal(o, o2)
