@@ -17,8 +17,8 @@
 //                                                                  mode warp 9 alone)
 // S = Q K^T accumulates in tensor memory; the softmax warps read it with tcgen05.ld, write the
 // bf16 probabilities back over the same columns and the PV product takes them from tensor memory.
-// Tensor memory with V: S0 S1 O0 O1, 128 columns each, at D = 128; three 128-column score buffers that both tiles go
-// round and two 64-column accumulators at D = 64.  The output leaves through shared memory by TMA.
+// Tensor memory with V: S0 S1 O0 O1, 128 columns each; at D = 64 with one item a thread block three 128-column score
+// buffers that both tiles go round and two 64-column accumulators.  The output leaves through shared memory by TMA.
 #pragma once
 #include "sm100_ptx.cuh"
 #include "softmax_steps.cuh"
@@ -99,9 +99,12 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   // With V at D = 64 the accumulators take 64 columns each, which leaves room for a third score buffer.  The score
   // tiles of both query tiles go round the three buffers (unit = step * tiles + tile, buffer = unit % 3): a tile's
   // next scores are computed while its softmax warps are still busy with the current ones.  What is left in the chain of
-  // a step is the softmax itself, (2, 16, 4096, 64): 0.217 -> 0.204 ms.  (The exponentials alone are 1536 clocks a step
-  // of both tiles, ex2 issuing once in 8 clocks a sub-partition, against 514 of products.)
-  constexpr bool ROT = HAS_V && D == 64;
+  // a step is the softmax itself, (2, 16, 4096, 64): 0.217 -> 0.207 ms; on clustered keys, where whole quarters are
+  // skipped and a step is shorter, (4, 24, 12345, 64) 4.99 -> 4.93 ms.  (The exponentials alone are 1536 clocks a step
+  // of both tiles, ex2 issuing once in 8 clocks a sub-partition, against 514 of products.)  Not in the
+  // persistent form, taken up to 1024 keys: there it is level from 512 keys on and costs 2 to 5 % below
+  // ((1, 40, 32768, 64) against 77 keys 0.113 ms without, 0.119 with it).
+  constexpr bool ROT = HAS_V && D == 64 && !PERSIST;
   constexpr uint32_t kColO = ROT ? 384 : 256, kOStride = ROT ? 64 : 128;
   constexpr bool TWO_ISS = (HAS_V && D == 128) || MODE == kML;   // one UMMA issuer warp per query tile ...
   constexpr int kTwoIssMinTiles = 64;                            // ... from 8192 keys on: with fewer the second
@@ -265,10 +268,10 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
     // scores), and an issuer that serves both tiles in turn reaches a tile's probabilities late whenever it is
     // busy with the other tile's waits and commits (C3 3.38 -> 3.20 ms).  The max / denominator mode gains the
     // same way (a freed score buffer is refilled at once: C3 2.32 -> 2.18 ms, C4 3.43 -> 3.36 ms).  With V at
-    // D = 64 the softmax, not the chain, bounds a step, two issuers are 1 % slower there and one warp serves
-    // both tiles, as in the token-mask mode and for key sequences under 8192.  (The gain depends on the data: on
-    // i.i.d. normal inputs, where no quarter of a score tile is ever skipped and the softmax step is longer, two
-    // issuers are level with one at 8192 keys and 1 % behind at 16384.)
+    // D = 64 one warp serves both tiles, whose units share the rotating buffers in one order (with one buffer a tile
+    // two issuers were 1 % slower), as in the token-mask mode and for key sequences under 8192.  (The gain depends on
+    // the data: on i.i.d. normal inputs, where no quarter of a score tile is ever skipped and the softmax step is
+    // longer, two issuers are level with one at 8192 keys and 1 % behind at 16384.)
     reg_dealloc<72>();
     const bool two_iss = TWO_ISS && p.n_kv_tiles >= kTwoIssMinTiles;
     const int t_lo = two_iss ? warp - 9 : 0, t_hi = two_iss ? t_lo + 1 : 2;
@@ -304,9 +307,11 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       for (int item = first_item; item < p.n_items && ok; item += item_step, ++it, g0 += n_tiles) {
         ok = mbar_wait_warp(bar(BAR_Q_FULL), it & 1, ab, p.err, 201);
         if constexpr (ROT) {
-          // Units in order: the product Q K^T of unit v + n_t + 1 follows P V of unit v, whose probabilities lie in
-          // the buffer that it overwrites (two tiles) or at most a step behind (one tile; never more than two
-          // steps' scores are out, so no barrier of a step parity completes twice unseen).
+          // Units in order (one item a thread block, so g0 = 0): the product Q K^T of unit v + n_t + 1 follows P V of
+          // unit v, whose probabilities lie in the buffer that it overwrites (two tiles) or at most a step behind (one
+          // tile; never more than two steps' scores are out, so no barrier of a step parity completes twice unseen).
+          // So the scores of step g are never published before P V of step g - 2 is done, which the softmax warps'
+          // wait for BAR_PV_DONE by the parity of step g - 1 relies on.
           const int n_t = __popc(tiles), t0 = (tiles & 1u) ? 0 : 1, n_units = n_tiles * n_t;
           auto qk_unit = [&](int v) {
             const int jj = (n_t == 2) ? v >> 1 : v, ti = (n_t == 2) ? v & 1 : 0;
@@ -315,7 +320,7 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
             if (ti == 0) ok = mbar_wait_warp(bar(BAR_K_FULL + ks), (g / kKSt) & 1, ab, p.err, 202);
             if (!ok) return;
             tc_fence_after();
-            issue_qk(t0 + ti, ks, ((g0 * n_t + v) % 3) * 128);
+            issue_qk(t0 + ti, ks, (v % 3) * 128);
             umma_commit_elect(bar(BAR_S_FULL + (t0 + ti) * 2 + (g & 1)));
             if (ti == n_t - 1) umma_commit_elect(bar(BAR_K_EMPTY + ks));
             if (v == n_units - 1) umma_commit_elect(bar(BAR_Q_EMPTY));
@@ -330,7 +335,7 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
             if (ok) ok = mbar_wait_warp(bar(BAR_P_FULL + t * 2 + (g & 1)), (g >> 1) & 1, ab, p.err, 205);
             if (!ok) break;
             tc_fence_after();
-            issue_pv(t, vs, jj > 0, ((g0 * n_t + v) % 3) * 128);
+            issue_pv(t, vs, jj > 0, (v % 3) * 128);
             umma_commit_elect(bar(BAR_PV_DONE + t));
             if (ti == n_t - 1) umma_commit_elect(bar(BAR_V_EMPTY + vs));
             if (jj == n_tiles - 1) umma_commit_elect(bar(BAR_O_FULL + t));
@@ -431,7 +436,7 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
         if (!ok) break;
         tc_fence_after();
         const uint32_t s_addr =
-            lane_base + (ROT ? ((tiles == 3u ? g * 2 + t : g) % 3) * 128 : HAS_V ? t * 128 : (t * 2 + b) * 128);
+            lane_base + (ROT ? ((tiles == 3u ? j * 2 + t : j) % 3) * 128 : HAS_V ? t * 128 : (t * 2 + b) * 128);
         const int key0 = tile_of(j) * 128;               // first key of this tile
         const int kv_left = p.kv_len - key0;             // valid keys in this tile
         const int valid0 = min(64, kv_left), valid1 = max(0, min(64, kv_left - 64));
@@ -488,7 +493,7 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
           }
         };
         const uint32_t o_addr = lane_base + kColO + t * kOStride;
-        if (HAS_V && D == 64 && j > 0 && kv_left >= 128)     // every tile but the first and a ragged last one
+        if (ROT && j > 0 && kv_left >= 128)     // every tile but the first and a ragged last one
           softmax_steady_step<D>(s_addr, s_addr, o_addr, c, st, mx0, mx1, quiet);
         else
           softmax_online_step<D, HAS_V>(s_addr, s_addr, o_addr, valid0, valid1, c, j == 0, st, mx0, mx1, nullptr, quiet);
