@@ -124,16 +124,31 @@ packed_to_index_kernel(const uint8_t* __restrict__ packed, int row_bytes, int* _
         chunk_total += t;
       }
       mine += incl[k] - c[k];
-      // The warp writes one word's entries at a time, a lane per bit: consecutive slots in one store, and a mask
-      // whose bits come in runs (whole words set next to empty ones) costs a trip per non-empty word instead of
-      // 32 trips of a single lane (3072 rows of 32768 bits, 5 % set in runs: 42 -> 29 us).
+      // Two ways to write the warp's entries.  Word by word, a lane per bit: a trip per non-empty word, its entries in one
+      // store -- for masks whose bits come in runs.  Or every lane its own word, bit by bit: as many trips as the fullest
+      // word has bits, each spread over about as many lines -- for scattered bits, a few in almost every word.
+      // 3072 rows of 32768 bits, us by words / by bits: set in runs, 5 % in runs of 256 20 / 37, 15 % in runs of 8 53 / 72;
+      // scattered, 1 % 35 / 16, 5 % 78 / 23, 10 % 89 / 31, 20 % 92 / 78, 50 % 93 / 291.  A trip by bits costs the more
+      // the more bits the words hold; most^2 / 5 trips by words are where the two meet.
       uint32_t todo = __ballot_sync(0xffffffffu, bits[k] != 0u);
-      while (todo) {
-        const int from = __ffs(todo) - 1;
-        todo &= todo - 1;
-        const uint32_t u = __shfl_sync(0xffffffffu, bits[k], from);
-        const int slot = __shfl_sync(0xffffffffu, mine, from) + __popc(u & ((1u << lane) - 1u));
-        if (((u >> lane) & 1u) && slot < list_stride) dst[slot] = 32 * (w0 + k * 256 + warp * 32 + from) + lane;
+      const int most = __reduce_max_sync(0xffffffffu, c[k]);
+      if (5 * __popc(todo) <= most * most) {
+        while (todo) {
+          const int from = __ffs(todo) - 1;
+          todo &= todo - 1;
+          const uint32_t u = __shfl_sync(0xffffffffu, bits[k], from);
+          const int slot = __shfl_sync(0xffffffffu, mine, from) + __popc(u & ((1u << lane) - 1u));
+          if (((u >> lane) & 1u) && slot < list_stride) dst[slot] = 32 * (w0 + k * 256 + warp * 32 + from) + lane;
+        }
+      } else {
+        const int w = w0 + k * 256 + tid;
+        uint32_t u = bits[k];
+        while (u) {
+          const int e = __ffs(u) - 1;
+          u &= u - 1;
+          if (mine < list_stride) dst[mine] = 32 * w + e;
+          ++mine;
+        }
       }
       off += chunk_total;
     }

@@ -154,3 +154,34 @@ def test_token_lists_by_way_of_bits(S, K, D):
     capi.check()
     used = torch.arange(idx.shape[-1], device="cuda") < cnt[..., None]
     assert torch.equal(num, cnt) and torch.equal(lists[used], idx[used]) and (lists[~used] == -7).all()
+
+
+@pytest.mark.parametrize("width,stride,n_valid", [(32768, 32768, 32760), (33000, 9000, 33000), (1096, 1096, 1090), (40, 40, 39)])
+@pytest.mark.parametrize("kind", ["runs", "scattered", "mixed", "one per word", "one word"])
+def test_packed_to_lists_of_runs_and_scattered_bits(kind, width, stride, n_valid):
+    """A warp writes its entries by words or by bits, whichever takes fewer trips: masks that go one way, the other way
+    and both ways in one row, lists that the entries overflow, and rows that are no whole number of words."""
+    from oracle import fgattn_oracle as orc
+    capi = _capi()
+    rows = 7
+    g = torch.Generator().manual_seed(width + len(kind))
+    runs = (torch.rand(rows, width // 8, generator=g) < 0.4).repeat_interleave(8, 1)
+    runs[:, width // 3: width // 2] = True
+    scattered = torch.rand(rows, width, generator=g) < torch.linspace(0, 0.3, rows)[:, None]
+    mask = {"runs": runs, "scattered": scattered, "mixed": torch.where(torch.arange(width) // 700 % 2 == 0, runs, scattered),
+            "one per word": (torch.arange(width) % 32 == torch.arange(rows)[:, None] * 5).contiguous(),
+            "one word": (torch.arange(width) // 32 == torch.arange(rows)[:, None]).contiguous()}[kind]
+    packed_np = orc.pack_mask(mask)
+    packed = torch.from_numpy(packed_np).cuda()
+    ridx, rcnt = orc.packedmask_to_indexmask(packed_np, n_valid=n_valid, stride=stride)
+    idx = torch.full((rows, stride), -1, dtype=torch.int32, device="cuda")
+    cnt = torch.full((rows,), -1, dtype=torch.int32, device="cuda")
+    capi.packedmask_to_indexmask(idx, cnt, packed, n_valid)
+    assert np.array_equal(cnt.cpu().numpy(), rcnt) and np.array_equal(idx.cpu().numpy(), ridx)
+    import fgattn_tk_cuda_b200.spattn  # noqa: F401  (registers torch.ops.cuda_attn)
+    lists, num = torch.full_like(idx, -7), torch.full_like(cnt, -7)
+    torch.ops.cuda_attn.packedmask_to_lists(lists, num, packed, n_valid)
+    capi.check()
+    used = np.arange(stride)[None, :] < rcnt[:, None]
+    got = lists.cpu().numpy()
+    assert np.array_equal(num.cpu().numpy(), rcnt) and np.array_equal(got[used], ridx[used]) and (got[~used] == -7).all()
