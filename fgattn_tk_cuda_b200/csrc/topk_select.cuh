@@ -354,9 +354,10 @@ topk_select_kernel(const float* __restrict__ scores, int s_stride, int n, int k,
   // ---- descending order.  The m collected entries are counted into 2048 bins of equal width over their range of
   // scores (a monotone map, so a larger bin holds smaller scores), every entry gets a slot in its bin, and inside a
   // bin -- a few entries -- an entry's place is the number of larger ones.  Five barriers where a bitonic sort of
-  // 4096 entries takes 78 passes over shared memory: 3276 of 32760 keys for 3072 rows, the whole selection with its
-  // attention 1.92 -> 1.61 ms.  The sort stays for scores that pile up in a few bins (equal or
-  // infinite ones), where counting inside the bins would be quadratic.
+  // 4096 entries takes 78 passes: 3276 of 32760 keys for 3072 rows, the whole selection 1.017 -> 0.569 ms (8192 keys
+  // 1.864 -> 1.001 ms, although the slots leave room for two rows on an SM instead of three).  The sort stays for scores
+  // that pile up in a few bins (equal or infinite ones, or one far above all others), where counting inside the bins
+  // would be quadratic: with kSelBinSort = 256 one score at 30 deviations takes 3.2 ms at 8192 keys, by the sort 1.55.
   const int m = (n_gt + s_ties <= k_pow2) ? n_gt + s_ties : k;
   const float f_hi = float_of_order_key(s_max), f_lo = float_of_order_key(kth);
   const float to_bin = float(kSelBins - 1) / (f_hi - f_lo);
@@ -420,9 +421,42 @@ topk_select_kernel(const float* __restrict__ scores, int s_stride, int n, int k,
     }
   }
 
-  // ---- bitonic sort, descending: the first k entries are the answer
-  for (int size = 2; size <= k_pow2; size <<= 1) {
-    for (int stride = size >> 1; stride > 0; stride >>= 1) {
+  // ---- bitonic sort, descending: the first k entries are the answer.  The passes of strides up to 32 stay inside groups
+  // of 64 entries: a warp takes a group through all of them in registers, two entries a lane, and only the passes
+  // of wider strides go through shared memory with a block barrier each (28 of 91 at 8192 entries).  Selections that end
+  // here pay for the histogram above too; with every pass through shared memory that made them slower than the sort
+  // alone: half of the scores equal, 3276 keys 1.234 -> 1.251 ms, now 1.156; 8192 keys 1.906 -> 2.102, now 1.826; one
+  // score at 30 deviations 1.017 -> 1.027, now 0.849, and 1.893 -> 1.990, now 1.550.
+  auto in_group = [&](int size_from, int size_to) {        // the passes of these sizes whose strides are 32 or less
+    for (int g = warp * 64; g < k_pow2; g += (kSelThreads / 32) * 64) {
+      unsigned long long x[2];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) x[h] = (g + 32 * h + lane < k_pow2) ? sel[g + 32 * h + lane] : 0ull;
+      for (int size = size_from; size <= size_to; size <<= 1) {
+        if (size >= 64) {
+          const bool desc = (g & size) == 0;
+          const unsigned long long a = x[0], b = x[1];
+          x[0] = ((a < b) == desc) ? b : a;
+          x[1] = ((a < b) == desc) ? a : b;
+        }
+        for (int stride = min(size, 32) >> 1; stride > 0; stride >>= 1) {
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const unsigned long long y = __shfl_xor_sync(0xffffffffu, x[h], stride);
+            const bool desc = ((g + 32 * h + lane) & size) == 0, upper = (lane & stride) != 0;
+            x[h] = ((x[h] < y) == (desc != upper)) ? y : x[h];
+          }
+        }
+      }
+#pragma unroll
+      for (int h = 0; h < 2; ++h)
+        if (g + 32 * h + lane < k_pow2) sel[g + 32 * h + lane] = x[h];
+    }
+    __syncthreads();
+  };
+  in_group(2, 64);                                         // (entries past the end of a short list count as zeros, the smallest)
+  for (int size = 128; size <= k_pow2; size <<= 1) {
+    for (int stride = size >> 1; stride > 32; stride >>= 1) {
       for (int t = tid; t < (k_pow2 >> 1); t += kSelThreads) {
         const int lo = 2 * t - (t & (stride - 1)), hi = lo + stride;
         const bool desc = (lo & size) == 0;
@@ -434,6 +468,7 @@ topk_select_kernel(const float* __restrict__ scores, int s_stride, int n, int k,
       }
       __syncthreads();
     }
+    in_group(size, size);
   }
   int* dst = idx + size_t(blockIdx.x) * list_stride;
   for (int i = tid; i < k; i += kSelThreads) dst[i] = int(~uint32_t(sel[i] & 0xffffffffull));

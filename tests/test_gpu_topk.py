@@ -120,7 +120,7 @@ def test_topk_argument_checks():
 def test_topk_order_of_any_distribution(kind, select_k):
     """The selected scores are put in order by counting where they spread over the bins and by the sort where they
     pile up: one key far above the rest, a few distinct values with many equal scores, scores on both sides of zero,
-    and scores that differ in their last bits only.  Equal scores: smaller key first."""
+    and scores in so small a range that the bin width has no inverse (by the sort).  Equal scores: smaller key first."""
     capi = _capi()
     S, D = 8320, 64
     g = torch.Generator().manual_seed(select_k)
@@ -146,3 +146,70 @@ def test_topk_order_of_any_distribution(kind, select_k):
     want = torch.sort(k[0, 0, :, 0].float(), descending=True, stable=True).indices[:select_k]
     assert torch.equal(idx[0, 0, 0, :select_k].cpu().long(), want)
     assert (idx[0, 0, 0, select_k:] == stride).all() and int(cnt) == select_k
+
+
+def _list_of_scores(f, scale_1, select_k, q0=1.0):
+    """The top-k list of one query block whose score of key i is q0 * f[i, 0] + scale_1 * f[i, 1], exactly."""
+    capi = _capi()
+    S, D = f.shape[0], 64
+    q = torch.zeros(1, 1, 128, D)
+    q[..., 0], q[..., 1] = q0, scale_1
+    k = torch.zeros(1, 1, S, D)
+    k[0, 0, :, :2] = f
+    q, k = q.to(torch.bfloat16), k.to(torch.bfloat16)
+    assert torch.equal(k[0, 0, :, :2].float(), f)
+    stride = 128 * ((select_k + 127) // 128)
+    idx = torch.full((1, 1, 1, stride), -1, dtype=torch.int32, device="cuda")
+    cnt = torch.full((1, 1, 1), -1, dtype=torch.int32, device="cuda")
+    capi.topk_indices(idx, cnt, q.cuda(), k.cuda(), select_k, blocksz=128, scale=1.0)
+    capi.check()
+    assert (idx[0, 0, 0, select_k:] == stride).all() and int(cnt) == select_k
+    return idx[0, 0, 0, :select_k].cpu().long()
+
+
+@pytest.mark.parametrize("select_k", [5, 33, 600, 5000])
+def test_topk_order_of_scores_a_few_ulps_apart(select_k):
+    """256 + n ulps, n in -256 .. 255: the range of the bins is 2^-14 of the scores, and 12 scores or so are equal each."""
+    S = 6200
+    n = torch.randint(-256, 256, (S,), generator=torch.Generator().manual_seed(select_k)).float()
+    got = _list_of_scores(torch.stack([torch.full((S,), 256.0), n], 1), 2.0 ** -15, select_k)
+    want = torch.sort(256.0 + n * 2.0 ** -15, descending=True, stable=True).indices[:select_k]
+    assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("pile", [63, 64, 65, 300])
+@pytest.mark.parametrize("S", [700, 2000])
+def test_topk_order_with_a_bin_at_its_limit(S, pile):
+    """Whole numbers from 0 to 2047 have a bin each (2047 over the range is one), and one of them occurs `pile` times:
+    counting takes 64 in a bin, the sort the rest.  Every key is selected, so that no other rule cuts the range."""
+    g = torch.Generator().manual_seed(S + pile)
+    x = torch.randperm(2046, generator=g)[: S - 2 - pile] + 1
+    x = torch.cat([torch.tensor([0, 2047]), x, torch.full((pile,), int(x[7]))])[torch.randperm(S, generator=g)]
+    got = _list_of_scores(torch.stack([x - x % 8, x % 8], 1).float(), 1.0, S)
+    assert torch.equal(got, torch.sort(x, descending=True, stable=True).indices)
+
+
+@pytest.mark.parametrize("k_to", [2, 16, 32, 64, 128, 256, 1024, 8192])
+@pytest.mark.parametrize("less", [0, 1])
+def test_topk_sort_of_every_size(k_to, less):
+    """Two values only, so that every selection ends in the sort: list lengths that fill its power of two or fall one
+    short of it, from less than a warp's group to the longest."""
+    select_k = max(1, k_to - less)
+    g = torch.Generator().manual_seed(k_to)
+    x = (torch.rand(9000, generator=g) < 0.4).float()
+    got = _list_of_scores(torch.stack([x, torch.zeros_like(x)], 1), 0.0, select_k)
+    assert torch.equal(got, torch.sort(x, descending=True, stable=True).indices[:select_k])
+
+
+@pytest.mark.parametrize("select_k", [4, 500, 1990, 2000])
+def test_topk_order_with_infinite_scores(select_k):
+    """Scores that overflow to infinity on either side, a few or half of them, and finite ones between (select_k up to
+    all of them: the range of the bins is then infinite on both sides)."""
+    S = 2000
+    g = torch.Generator().manual_seed(select_k)
+    x = torch.randn(S, generator=g).to(torch.bfloat16).float()
+    x[torch.randperm(S, generator=g)[:7]] = 2.0 ** 127
+    x[torch.randperm(S, generator=g)[:9]] = -2.0 ** 127
+    got = _list_of_scores(torch.stack([x, torch.zeros_like(x)], 1), 0.0, select_k, q0=4.0)
+    want = torch.sort(4.0 * x, descending=True, stable=True).indices[:select_k]
+    assert torch.equal(got, want)
