@@ -102,7 +102,7 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   // a step is the softmax itself, (2, 16, 4096, 64): 0.217 -> 0.207 ms; on clustered keys, where whole quarters are
   // skipped and a step is shorter, (4, 24, 12345, 64) 4.99 -> 4.93 ms.  (The exponentials alone are 1536 clocks a step
   // of both tiles, ex2 issuing once in 8 clocks a sub-partition, against 514 of products.)  Not in the
-  // persistent form, taken up to 1024 keys: there it is level from 512 keys on and costs 2 to 5 % below
+  // persistent form, taken up to 1024 keys: there it gives 2 % at 1000 keys, nothing at 512 and costs 2 to 5 % below
   // ((1, 40, 32768, 64) against 77 keys 0.113 ms without, 0.119 with it).
   constexpr bool ROT = HAS_V && D == 64 && !PERSIST;
   constexpr uint32_t kColO = ROT ? 384 : 256, kOStride = ROT ? 64 : 128;
