@@ -291,7 +291,9 @@ int launch_sparse(void* o, const void* q, const void* k, const void* v, const in
   int sms = 0;
   r = sm_count(&sms);
   if (r) return r;
-  if (workspace && n_units * p.quads > sms) {       // (with a thread block per SM or fewer all items start at once)
+  // (With a thread block per SM or fewer the order changes nothing on an idle GPU.  Beside a kernel of another stream
+  // that holds SMs the items start as those come free, in storage order.)
+  if (workspace && n_units * p.quads > sms) {
     // CTA order: units in groups whose K/V (<= 64 MiB) stays in L2, inside a group longest lists first
     const size_t kv_bytes_per_unit = size_t(4) * kv_rows * D;
     int group = int(std::max<size_t>(1, (size_t(64) << 20) / kv_bytes_per_unit));
@@ -461,7 +463,7 @@ int token_mask_launch(int* booleanmask, uint32_t* bits, float threshold, int mas
   int sms = 0;
   r = sm_count(&sms);
   if (r) return r;
-  if (kb_indices && workspace && batch * heads * ((seq + 255) / 256) > sms) {     // fewer items all start at once
+  if (kb_indices && workspace && batch * heads * ((seq + 255) / 256) > sms) {     // (no order for fewer items than SMs)
     // thread-block order: inside groups of units the items (four 64-row query blocks) with the longest
     // lists first.  Large groups balance better than small ones keep K in L2 (measured at
     // (1,12,32760,128): storage order 0.58 ms, 3 heads per group 0.57, 6: 0.50, all 12: 0.40).
@@ -622,7 +624,7 @@ int fgattn_sp_attn(void* o, const void* q, const void* k, const void* v, const i
   int sms = 0;
   r = sm_count(&sms);
   if (r) return r;
-  if (workspace && n_units * p.pairs > sms) {       // (with a thread block per SM or fewer all items start at once)
+  if (workspace && n_units * p.pairs > sms) {       // (no order for fewer items than SMs)
     // thread-block order: inside groups of units, longest lists first.  The row gather gains little from
     // L2 residency of K/V, and large groups balance better (measured at (1,12,32760,128): 0.90 ms in
     // storage order, 0.77 ms with 4 heads per group, 0.55 ms with all 12), so groups span up to 256 MiB of K/V.
@@ -874,8 +876,8 @@ int launch_sparse_persistent(bool renorm, void* o, const void* q, const void* k,
   group_heads = std::max(1, std::min(group_heads, n_units));
   const int n_groups = std::max(1, n_units / group_heads);
   if (p.n_items <= sms) {
-    // Every item has a thread block of its own and all of them start at once: neither a queue nor an order
-    // changes anything, so the launch that makes them (one block, 3-10 us) is left out.
+    // Every item has a thread block of its own and, on an idle GPU, all of them start at once: neither a queue nor an
+    // order changes anything, so the launch that makes them (one block, 3-10 us) is left out.
     p.order = nullptr;
     if (renorm) FG_CUDA(cudaMemsetAsync(p.redo, 0, size_t(p.n_items) * sizeof(int), st));
   } else {

@@ -197,7 +197,10 @@ def test_thread_block_order_with_several_head_groups(group):
 
 
 def _order_case(capi, orc):
-    B, H, S, D = 1, 5, 1500, 64
+    B, S, D = 1, 1500, 64
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    H = sms // 6 + 2
+    assert B * H * ((S + 255) // 256) > sms            # with fewer items than SMs there is no order
     nqb = nkb = (S + 63) // 64
     g = torch.Generator().manual_seed(77)
     q, k, v = (torch.randn(B, H, S, D, generator=g).to(torch.bfloat16).cuda() for _ in range(3))
@@ -225,6 +228,47 @@ def _order_case(capi, orc):
     capi.check()
     assert torch.equal(t_st, t_or)
     assert torch.isfinite(t_or.float()).all()
+
+
+@pytest.mark.parametrize("group", [3, 0])
+def test_token_mask_order_with_bucketed_lengths(group):
+    """The longest-first order of the listed token mask, more items than SMs and enough key blocks that four lists
+    share length buckets: the same mask as in storage order, as int32 and as bits."""
+    capi = _capi()
+    import fgattn_tk_cuda_b200.spattn  # noqa: F401  (registers torch.ops.cuda_attn)
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B, S, K, D = 1, 900, 16500, 64
+    H = sms // 4 + 2
+    nqb, nkb = (S + 63) // 64, (K + 63) // 64
+    assert H * ((S + 255) // 256) > sms and 4 * nkb > 1024
+    g = torch.Generator().manual_seed(5)
+    q = torch.randn(B, H, S, D, generator=g).to(torch.bfloat16).cuda()
+    k = torch.randn(B, H, K, D, generator=g).to(torch.bfloat16).cuda()
+    bm = torch.rand(B, H, nqb, nkb, generator=g) < torch.rand(B, H, nqb, 1, generator=g)
+    bm[:, 1] = False
+    cnt = bm.sum(-1, dtype=torch.int32)
+    idx = torch.sort(torch.where(bm, torch.arange(nkb), nkb), -1).values.to(torch.int32)
+    s_pad = 128 * ((S + 127) // 128)
+    m = torch.empty(B, H, 1, s_pad, device="cuda")
+    l = torch.empty_like(m)
+    capi.maxq_denom(m, l, q, k)
+    stride = 128 * ((K + 127) // 128)
+    want = torch.full((B, H, s_pad // 128, stride), 9, dtype=torch.int32, device="cuda")
+    got = torch.full_like(want, 9)
+    bits = torch.full((B, H, s_pad // 128, stride // 8), 0xAA, dtype=torch.uint8, device="cuda")
+    capi.set_tuning("group_heads", group)
+    try:
+        capi.booleanmask_128_listed(want, m, l, q, k, 1e-4, idx.cuda(), cnt.cuda(), ordered=False)
+        capi.booleanmask_128_listed(got, m, l, q, k, 1e-4, idx.cuda(), cnt.cuda())
+        torch.ops.cuda_attn.packedmask_128_listed(bits, m, l, q, k, 1e-4, idx.cuda(), cnt.cuda())
+        capi.check()
+    finally:
+        capi.set_tuning("group_heads", -1)
+    assert torch.equal(got, want)
+    assert not want[:, 1].any() and 0.0 < want.float().mean().item() < 0.9
+    unpacked = torch.empty_like(want)
+    capi.unpack_mask(unpacked, bits)
+    assert torch.equal(unpacked, (want > 0).int())
 
 
 @pytest.mark.parametrize("S,D,kv", [(1000, 128, None), (1536, 64, 1400)])

@@ -188,3 +188,60 @@ def test_block_route_large_scores_rerun():
         capi.set_tuning("token_block_route", -1)
     _close(o, ref)
     assert _routes(capi, ws, B, H, S).sum() == 4
+
+
+def test_block_route_with_more_items_than_sms():
+    """The queue of the block route with fewer thread blocks than items, of which some are left to the row gather."""
+    from oracle import fgattn_oracle as orc
+    capi = _capi()
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    B, S, D = 1, 1500, 64
+    nb, stride = (S + 127) // 128, 128 * ((S + 127) // 128)
+    H = sms // nb + 2
+    assert H * nb > sms
+    g = torch.Generator().manual_seed(8)
+    q, k, v = (torch.randn(B, H, S, D, generator=g).to(torch.bfloat16) for _ in range(3))
+    keep = torch.rand(B, H, nb, 1, generator=g)                 # list lengths from a few blocks to all
+    blocks = torch.rand(B, H, nb, (S + 63) // 64, generator=g) < keep
+    tm = blocks.repeat_interleave(64, dim=-1)[..., :S] & (torch.rand(B, H, nb, S, generator=g) < 0.9)
+    tm[:, :, ::5] = torch.rand(B, H, (nb + 4) // 5, S, generator=g) < 0.05
+    idx, cnt = _lists_from_mask(tm, stride)
+    qc, kc, vc, idxc, cntc = q.cuda(), k.cuda(), v.cuda(), idx.cuda(), cnt.cuda()
+    ws = torch.empty(capi.sp_attn_token_workspace_bytes(B, H, S, S), dtype=torch.uint8, device="cuda")
+    o, o_g = torch.full_like(qc, float("nan")), torch.full_like(qc, float("nan"))
+    capi.set_tuning("token_block_route", 1)
+    try:
+        capi.sp_attn(o, qc, kc, vc, idxc, cntc, workspace=ws)
+        capi.check()
+    finally:
+        capi.set_tuning("token_block_route", -1)
+    taken = _routes(capi, ws, B, H, S)
+    assert not taken[:, ::5].any() and taken.float().mean().item() > 0.6
+    capi.sp_attn(o_g, qc, kc, vc, idxc, cntc, block_route=False)
+    capi.check()
+    assert (o.float() - o_g.float()).abs().max().item() <= 1.6e-2
+    _close(o[:, :3], orc.sp_attn_tokens(q[:, :3], k[:, :3], v[:, :3], idx[:, :3], cnt[:, :3], 128))
+
+
+@pytest.mark.parametrize("S,D", [(1, 128), (31, 64), (33, 128), (129, 64), (160, 128), (257, 64), (385, 128)])
+def test_output_rows_at_the_edges(S, D):
+    """The output leaves from the query tile's own buffer in boxes of 32 rows: sequences that end inside a box, at its
+    edge, in either query tile, lists of one step and of several, an empty one.  Nothing past the last row of the last
+    head may be written, nothing of a head's rows by the one before it."""
+    from oracle import fgattn_oracle as orc
+    capi = _capi()
+    B, H, K = 1, 3, 700
+    g = torch.Generator().manual_seed(S)
+    q = torch.randn(B, H, S, D, generator=g).to(torch.bfloat16)
+    k, v = (torch.randn(B, H, K, D, generator=g).to(torch.bfloat16) for _ in range(2))
+    nb, stride = (S + 127) // 128, 768
+    tm = torch.rand(B, H, nb, K, generator=g) < torch.tensor([0.1, 0.9, 0.4])[None, :, None, None]
+    tm[0, 2, -1] = False
+    idx, cnt = _lists_from_mask(tm, stride)
+    n = B * H * S * D
+    buf = torch.full((n + 40 * D,), 7.0, device="cuda", dtype=torch.bfloat16)
+    o = buf[:n].view(B, H, S, D)
+    capi.sp_attn(o, q.cuda(), k.cuda(), v.cuda(), idx.cuda(), cnt.cuda())
+    capi.check()
+    _close(o, orc.sp_attn_tokens(q, k, v, idx, cnt, 128))
+    assert torch.all(buf[n:] == 7.0)

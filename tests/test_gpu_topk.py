@@ -213,3 +213,26 @@ def test_topk_order_with_infinite_scores(select_k):
     got = _list_of_scores(torch.stack([x, torch.zeros_like(x)], 1), 0.0, select_k, q0=4.0)
     want = torch.sort(4.0 * x, descending=True, stable=True).indices[:select_k]
     assert torch.equal(got, want)
+
+
+@pytest.mark.parametrize("select_k", [4, 500, 2000])
+def test_topk_with_nan_scores(select_k):
+    """NaN scores have no order, but the list stays one of distinct keys, with the others in descending order."""
+    S = 2000
+    x = torch.randn(S, generator=torch.Generator().manual_seed(select_k)).to(torch.bfloat16).float()
+    bad = torch.zeros(S, dtype=torch.bool)
+    bad[::97] = True
+    k = torch.zeros(1, 1, S, 64)
+    k[0, 0, :, 0] = torch.where(bad, torch.tensor(float("nan")), x)
+    q = torch.zeros(1, 1, 128, 64)
+    q[..., 0] = 1.0
+    idx = torch.full((1, 1, 1, 2048), -1, dtype=torch.int32, device="cuda")
+    cnt = torch.full((1, 1, 1), -1, dtype=torch.int32, device="cuda")
+    capi = _capi()
+    capi.topk_indices(idx, cnt, q.to(torch.bfloat16).cuda(), k.to(torch.bfloat16).cuda(), select_k, blocksz=128, scale=1.0)
+    capi.check()
+    got = idx[0, 0, 0, :select_k].cpu().long()
+    assert got.min() >= 0 and got.max() < S and got.unique().numel() == select_k and int(cnt) == select_k
+    numbers = got[~bad[got]]
+    want = torch.sort(torch.where(bad, torch.tensor(float("-inf")), x), descending=True, stable=True).indices
+    assert torch.equal(numbers, want[: numbers.numel()])
