@@ -260,7 +260,8 @@ topk_select_kernel(const float* __restrict__ scores, int s_stride, int n, int k,
   }
   __syncthreads();
 
-  // ---- narrow [lo, hi] around the k-th largest key
+  // ---- narrow [lo, hi] around the k-th largest key.  hi - lo < 2^shift after a sweep, so shift goes from 21 at most to
+  // 10 to 0: three sweeps at most.
   while (true) {
     const uint32_t lo = s_lo, hi = s_hi;
     const int rem = s_rem;
@@ -293,7 +294,7 @@ topk_select_kernel(const float* __restrict__ scores, int s_stride, int n, int k,
         }
         const uint32_t nlo = lo + (uint32_t(b0 + b) << shift);
         s_lo = nlo;
-        s_hi = (shift == 0) ? nlo : min(hi, nlo + ((1u << shift) - 1u));
+        s_hi = nlo + min(hi - nlo, (1u << shift) - 1u);          // (the keys of NaNs reach 2^32 - 1: no wrap)
         s_rem = r;
         s_ties = hist[b0 + b];
       }
