@@ -57,7 +57,7 @@ template <int D>
 struct DenseCfg {
   static constexpr int kHalves = D / 64;                 // 128-byte column groups per row
   static constexpr int kTileBytes = 128 * D * 2;         // one 128-row tile of Q, K or V
-  static constexpr int kKStages = (D == 64) ? 3 : 2, kVStages = kKStages;
+  static constexpr int kKStages = 2, kVStages = 2;
   static constexpr int kOffQ = 0;
   static constexpr int kOffK = 2 * kTileBytes;
   static constexpr int kOffV = kOffK + kKStages * kTileBytes;
