@@ -17,8 +17,8 @@
 //                                                                  mode warp 9 alone)
 // S = Q K^T accumulates in tensor memory; the softmax warps read it with tcgen05.ld, write the
 // bf16 probabilities back over the same columns and the PV product takes them from tensor memory.
-// Tensor memory with V: S0 S1 O0 O1, 128 columns each; at D = 64 with one item a thread block three 128-column score
-// buffers that both tiles go round and two 64-column accumulators.  The output leaves through shared memory by TMA.
+// Tensor memory with V: S0 S1 O0 O1, 128 columns each; with rotating score buffers (ROT, at D = 64) three 128-column
+// ones that both tiles go round and two 64-column accumulators.  The output leaves through shared memory by TMA.
 #pragma once
 #include "sm100_ptx.cuh"
 #include "softmax_steps.cuh"
@@ -86,7 +86,7 @@ enum : int {
   BAR_COUNT = 34
 };
 
-template <int D, int MODE, bool BLOCKMAX, bool PERSIST>
+template <int D, int MODE, bool BLOCKMAX, bool PERSIST, bool ROT>
 __global__ void __launch_bounds__(384, 1)
 dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__ CUtensorMap mk,
                   const __grid_constant__ CUtensorMap mv, const __grid_constant__ CUtensorMap mo, const DenseParams p) {
@@ -101,10 +101,9 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   // next scores are computed while its softmax warps are still busy with the current ones.  What is left in the chain of
   // a step is the softmax itself, (2, 16, 4096, 64): 0.217 -> 0.207 ms; on clustered keys, where whole quarters are
   // skipped and a step is shorter, (4, 24, 12345, 64) 4.99 -> 4.93 ms.  (The exponentials alone are 1536 clocks a step
-  // of both tiles, ex2 issuing once in 8 clocks a sub-partition, against 514 of products.)  Not in the
-  // persistent form, taken up to 1024 keys: there it gives 2 % at 1000 keys, nothing at 512 and costs 2 to 5 % below
-  // ((1, 40, 32768, 64) against 77 keys 0.113 ms without, 0.119 with it).
-  constexpr bool ROT = HAS_V && D == 64 && !PERSIST;
+  // of both tiles, ex2 issuing once in 8 clocks a sub-partition, against 514 of products.)  The persistent form
+  // rotates where an item is long enough (kOneBufferMaxKeyTiles of the launcher).
+  static_assert(!ROT || (HAS_V && D == 64), "room for a third score buffer");
   constexpr uint32_t kColO = ROT ? 384 : 256, kOStride = ROT ? 64 : 128;
   constexpr bool TWO_ISS = (HAS_V && D == 128) || MODE == kML;   // one UMMA issuer warp per query tile ...
   constexpr int kTwoIssMinTiles = 64;                            // ... from 8192 keys on: with fewer the second
@@ -307,7 +306,7 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       for (int item = first_item; item < p.n_items && ok; item += item_step, ++it, g0 += n_tiles) {
         ok = mbar_wait_warp(bar(BAR_Q_FULL), it & 1, ab, p.err, 201);
         if constexpr (ROT) {
-          // Units in order (one item a thread block, so g0 = 0): the product Q K^T of unit v + n_t + 1 follows P V of
+          // Units in order, round the buffers from item to item: the product Q K^T of unit v + n_t + 1 follows P V of
           // unit v, whose probabilities lie in the buffer that it overwrites (two tiles) or at most a step behind (one
           // tile; never more than two steps' scores are out, so no barrier of a step parity completes twice unseen).
           // So the scores of step g are never published before P V of step g - 2 is done, which the softmax warps'
@@ -320,7 +319,7 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
             if (ti == 0) ok = mbar_wait_warp(bar(BAR_K_FULL + ks), (g / kKSt) & 1, ab, p.err, 202);
             if (!ok) return;
             tc_fence_after();
-            issue_qk(t0 + ti, ks, (v % 3) * 128);
+            issue_qk(t0 + ti, ks, ((g0 * n_t + v) % 3) * 128);
             umma_commit_elect(bar(BAR_S_FULL + (t0 + ti) * 2 + (g & 1)));
             if (ti == n_t - 1) umma_commit_elect(bar(BAR_K_EMPTY + ks));
             if (v == n_units - 1) umma_commit_elect(bar(BAR_Q_EMPTY));
@@ -335,7 +334,7 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
             if (ok) ok = mbar_wait_warp(bar(BAR_P_FULL + t * 2 + (g & 1)), (g >> 1) & 1, ab, p.err, 205);
             if (!ok) break;
             tc_fence_after();
-            issue_pv(t, vs, jj > 0, (v % 3) * 128);
+            issue_pv(t, vs, jj > 0, ((g0 * n_t + v) % 3) * 128);
             umma_commit_elect(bar(BAR_PV_DONE + t));
             if (ti == n_t - 1) umma_commit_elect(bar(BAR_V_EMPTY + vs));
             if (jj == n_tiles - 1) umma_commit_elect(bar(BAR_O_FULL + t));
@@ -436,7 +435,7 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
         if (!ok) break;
         tc_fence_after();
         const uint32_t s_addr =
-            lane_base + (ROT ? ((tiles == 3u ? j * 2 + t : j) % 3) * 128 : HAS_V ? t * 128 : (t * 2 + b) * 128);
+            lane_base + (ROT ? ((tiles == 3u ? g * 2 + t : g) % 3) * 128 : HAS_V ? t * 128 : (t * 2 + b) * 128);
         const int key0 = tile_of(j) * 128;               // first key of this tile
         const int kv_left = p.kv_len - key0;             // valid keys in this tile
         const int valid0 = min(64, kv_left), valid1 = max(0, min(64, kv_left - 64));

@@ -150,10 +150,10 @@ int sm_count(int* out) {
 // One launch of the dense family over heads [bh0, bh0 + nbh).  Work item = pair of 128-row query tiles
 // of one unit.  PERSIST: one CTA per SM walks the items (pays off when an item has few key tiles, so
 // that the CTA prologue and the first loads would otherwise dominate); else one CTA per item.
-template <int D, int MODE, bool BLOCKMAX, bool PERSIST>
+template <int D, int MODE, bool BLOCKMAX, bool PERSIST, bool ROT>
 int launch_dense_k(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorMap& mv, const CUtensorMap& mo,
                    const fg::DenseParams& p, int ctas, cudaStream_t st) {
-  auto kern = fg::dense_attn_kernel<D, MODE, BLOCKMAX, PERSIST>;
+  auto kern = fg::dense_attn_kernel<D, MODE, BLOCKMAX, PERSIST, ROT>;
   int r = set_smem(kern, fg::DenseCfg<D>::kSmemBytes);
   if (r) return r;
   kern<<<dim3(ctas, 1, 1), 384, fg::DenseCfg<D>::kSmemBytes, st>>>(mq, mk, mv, mo, p);
@@ -162,6 +162,9 @@ int launch_dense_k(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorM
 }
 
 constexpr int kPersistMaxKeyTiles = 8;     // persistent CTAs up to 1024 keys
+// Persistent CTAs at D = 64: the score buffers rotate above 512 keys.  16384 rows of 24 heads, one buffer a tile against
+// rotating ones: 77 keys 40.7 / 41.7 us, 128 keys 37.1 / 39.2, 512 keys level, 1000 keys 170.7 / 166.7
+constexpr int kOneBufferMaxKeyTiles = 4;
 // The max / denominator pass alone stays persistent up to 2048 keys: measured against its one-item kernel
 // (maxq_pass.cuh) at 32768 queries x 40 heads, D = 128 / 64: 1280 keys 16 / 12 % faster, 1536 keys 13 / 6 %,
 // 2048 keys 10 / 4 %, 3072 keys level / 1 % slower
@@ -185,6 +188,7 @@ int launch_dense_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorM
   fg::DenseParams pp = p;
   pp.n_pairs = (p.S + 255) / 256;
   pp.n_items = pp.n_pairs * nbh;
+  constexpr bool rot = D == 64 && (MODE == fg::kFull || MODE == fg::kFullML);
   if constexpr (MODE != fg::kTokenMask && !BLOCKMAX) {
     const int persist_env = env_dense_persist();
     const bool persist = persist_env >= 0 ? persist_env != 0
@@ -193,7 +197,12 @@ int launch_dense_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorM
       int sms = 0;
       int r = sm_count(&sms);
       if (r) return r;
-      return launch_dense_k<D, MODE, BLOCKMAX, true>(mq, mk, mv, mo, pp, pp.n_items < sms ? pp.n_items : sms, st);
+      const int ctas = pp.n_items < sms ? pp.n_items : sms;
+      if constexpr (rot) {
+        if (p.n_kv_tiles > kOneBufferMaxKeyTiles)
+          return launch_dense_k<D, MODE, BLOCKMAX, true, true>(mq, mk, mv, mo, pp, ctas, st);
+      }
+      return launch_dense_k<D, MODE, BLOCKMAX, true, false>(mq, mk, mv, mo, pp, ctas, st);
     }
   }
   // One thread block per item.  When the last wave of thread blocks would be less than half full, its items
@@ -217,7 +226,7 @@ int launch_dense_t(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorM
     if (wide_env != 0 && !(MODE == fg::kTokenMask && p.kb_idx != nullptr))
       return launch_maxq_wide<D, BLOCKMAX, MODE == fg::kTokenMask>(mq, mk, pp, ctas, st);
   }
-  return launch_dense_k<D, MODE, BLOCKMAX, false>(mq, mk, mv, mo, pp, ctas, st);
+  return launch_dense_k<D, MODE, BLOCKMAX, false, rot>(mq, mk, mv, mo, pp, ctas, st);
 }
 
 struct DenseSetup {

@@ -64,7 +64,8 @@ def test_dense_family(B, H, S, Skv, D, kv):
 
 @pytest.mark.parametrize("B,H,S,Skv,D,kv", [(1, 4, 15000, 300, 64, None), (2, 3, 13000, 1024, 128, 1000),
                                              (1, 5, 9999, 128, 128, None), (1, 4, 13000, 500, 64, None),
-                                             (1, 4, 13000, 640, 64, 577), (1, 4, 13000, 77, 64, None)])
+                                             (1, 4, 13000, 640, 64, 577), (1, 4, 13000, 77, 64, None),
+                                             (1, 4, 13000, 1000, 64, None)])
 def test_few_keys_many_query_tiles(B, H, S, Skv, D, kv):
     """Up to 1024 keys the dense family runs persistent CTAs that walk several (unit, query tile pair)
     items each; these shapes have more items than the GPU has SMs."""
