@@ -1,6 +1,6 @@
 // Sparse attention over key-TOKEN lists at the reference granularity (128-row query blocks).
 // For each query block the listed K/V rows are gathered 128 at a time into swizzled shared-memory
-// tiles (16-byte cp.async per chunk, whole rows per warp-wide copy, fifteen gather warps), and the flash-attention step over the
+// tiles (16-byte cp.async per chunk, whole rows per warp-wide copy, seven gather warps), and the flash-attention step over the
 // gathered keys runs on tcgen05 with an online (renormalising) softmax.  A CTA runs two query
 // blocks ("slots") against one tensor pipe; their K/V tiles share one ring in consumption order.
 // List entries >= the number of key rows, and slots past the count, are masked out.
@@ -33,7 +33,13 @@ struct TokenCfg {
   static constexpr int kHalves = D / 64;
   static constexpr int kTileBytes = 128 * D * 2;
   static constexpr int kStages = (D == 128) ? 4 : 8;
-  static constexpr int kGatherWarps = 15;                 // the copies a warp can keep in flight are the limit
+  // Seven gather warps keep up: the copies wait for nothing but free stages (a bare gather of the same rows by eight warps
+  // runs at 19 TB/s, three times what this kernel draws).  What bounds a step is the softmax and the round trip through
+  // the products, so the registers go to the softmax warps (208), which hold a row's 128 scores and read them from tensor
+  // memory once.  With fifteen gather warps the softmax had 152 and read them twice, 32 at a time: 12 heads of 32760 rows,
+  // D = 128, 3276 keys of every block 0.896 -> 0.752 ms, threshold lists (1626 on average) 0.474 -> 0.414; D = 64 0.757 ->
+  // 0.724 and 0.402 -> 0.378 (both with the list entries requested ahead, see the softmax warps).
+  static constexpr int kGatherWarps = 7;
   static constexpr int kGatherThreads = 32 * kGatherWarps;
   static constexpr int kThreads = 32 * (8 + 1 + kGatherWarps);   // 8 softmax warps, the UMMA issuer, the gather warps
   static constexpr int kOffQ = 0;
@@ -51,89 +57,6 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N>
 __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory"); }
 
-
-// Online softmax over one 128-column score tile in two passes of 32-column quarters, so that a thread
-// never holds more than 32 scores: pass 1 finds the row maximum over the live columns (colmask: 4
-// words, bit set = live), pass 2 re-reads the scores, writes the bf16 probabilities over the first 64
-// columns of the same tile and adds up the row sum.  The accumulator row is rescaled lazily (2^8 rule).
-template <int D>
-__device__ __forceinline__ void softmax_online_quarters(uint32_t s_addr, uint32_t o_addr, float c, bool first,
-                                                        OnlineState& st, const uint32_t (&colmask)[4]) {
-  float mx = -INFINITY;
-#pragma unroll
-  for (int w = 0; w < 4; ++w) {
-    const uint32_t mw = colmask[w];
-    if (mw == 0u) continue;                              // warp-uniform: no live column in this quarter
-    uint32_t r[32];
-    tmem_ld32(s_addr + w * 32, r);
-    tmem_ld_wait();
-    if (mw == 0xffffffffu) {   // all but a list's last step: no column tests ((1,12,32760,128) at 5 %: 0.621 -> 0.594 ms)
-      mx = fmaxf(mx, quarter_max(r));
-      continue;
-    }
-    float c0 = -INFINITY, c1 = -INFINITY, c2 = -INFINITY, c3 = -INFINITY;
-#pragma unroll
-    for (int i = 0; i < 32; i += 4) {
-      c0 = fmaxf(c0, ((mw >> i) & 1u) ? __uint_as_float(r[i]) : -INFINITY);
-      c1 = fmaxf(c1, ((mw >> (i + 1)) & 1u) ? __uint_as_float(r[i + 1]) : -INFINITY);
-      c2 = fmaxf(c2, ((mw >> (i + 2)) & 1u) ? __uint_as_float(r[i + 2]) : -INFINITY);
-      c3 = fmaxf(c3, ((mw >> (i + 3)) & 1u) ? __uint_as_float(r[i + 3]) : -INFINITY);
-    }
-    mx = fmaxf(mx, fmaxf(fmaxf(c0, c1), fmaxf(c2, c3)));
-  }
-  st.m_true = fmaxf(st.m_true, mx);
-  const float ms = mx * c;
-  const bool grow = ms > st.m_used + 8.0f;
-  if (__any_sync(0xffffffffu, grow)) {
-    const float alpha = grow ? ex2(st.m_used - ms) : 1.0f;
-    if (grow) st.m_used = ms;
-    st.l *= alpha;
-    if (!first) {
-#pragma unroll
-      for (int cc = 0; cc < D / 32; ++cc) {
-        uint32_t o[32];
-        tmem_ld32(o_addr + cc * 32, o);
-        tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * alpha);
-        tmem_st32(o_addr + cc * 32, o);
-      }
-    }
-  }
-  const float neg_m = -st.m_used;
-  float sum0 = 0.f, sum1 = 0.f;
-#pragma unroll
-  for (int w = 0; w < 4; ++w) {
-    const uint32_t mw = colmask[w];
-    uint32_t pk[16];
-    if (mw != 0u) {
-      uint32_t r[32];
-      tmem_ld32(s_addr + w * 32, r);
-      tmem_ld_wait();
-      auto probs = [&](const bool masked) {
-#pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float p0 = ex2(fmaf(__uint_as_float(r[i]), c, neg_m));
-          float p1 = ex2(fmaf(__uint_as_float(r[i + 1]), c, neg_m));
-          if (masked && !((mw >> i) & 1u)) p0 = 0.f;
-          if (masked && !((mw >> (i + 1)) & 1u)) p1 = 0.f;
-          sum0 += p0;
-          sum1 += p1;
-          pk[i >> 1] = pack_bf16(p0, p1);
-        }
-      };
-      if (mw == 0xffffffffu) probs(false);
-      else probs(true);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 16; ++i) pk[i] = 0u;
-    }
-    // quarter w's probabilities land on columns 16w .. 16w+15, all of them already consumed
-    tmem_st16(s_addr + w * 16, pk);
-  }
-  st.l += sum0 + sum1;
-  tmem_st_wait();
-}
 
 template <int D>
 __global__ void __launch_bounds__(TokenCfg<D>::kThreads, 1)
@@ -186,25 +109,19 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  // per-slot list and number of 128-token steps
-  int cnt[2], nst[2];
-  const int* lst[2];
-#pragma unroll
-  for (int t = 0; t < 2; ++t) {
+  // per-slot list length and number of 128-token steps; slot t's list starts at lst + t * mask_stride
+  const int* const lst = p.kv_idx + (size_t(bh) * p.nqb + (q0 >> 7)) * p.mask_stride;
+  auto list_length = [&](int t) {
     const int qb = (q0 >> 7) + t;
-    cnt[t] = 0;
-    lst[t] = p.kv_idx;
-    if (qb < p.nqb && !skip[t]) {
-      cnt[t] = max(0, min(p.kv_cnt[size_t(bh) * p.nqb + qb], p.mask_stride));
-      lst[t] = p.kv_idx + (size_t(bh) * p.nqb + qb) * p.mask_stride;
-    }
-    nst[t] = (cnt[t] + 127) >> 7;
-  }
-  const int n_max = max(nst[0], nst[1]);
+    const bool none = qb >= p.nqb || (t ? skip[1] : skip[0]);
+    return none ? 0 : max(0, min(p.kv_cnt[size_t(bh) * p.nqb + qb], p.mask_stride));
+  };
+  const int cnt0 = list_length(0), cnt1 = list_length(1);
+  const int nst0 = (cnt0 + 127) >> 7, nst1 = (cnt1 + 127) >> 7, n_max = max(nst0, nst1);
 
   if (warp == 8 || warp >= 10) {
     // ------------------------------------------------------------------ gather producers
-    reg_dealloc<40>();
+    reg_dealloc<48>();
     if (warp == 8 && lane == 0) {
       tma_prefetch_desc(&mq);
       tma_prefetch_desc(&mo);
@@ -215,25 +132,23 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
                       bh);
     }
     __syncwarp();
-    const int gw = (warp == 8) ? 0 : warp - 9;                         // gather warp 0..14
+    const int gw = (warp == 8) ? 0 : warp - 9;                         // gather warp 0..6
     constexpr int kChunksPerRow = D / 8;                               // 16-byte chunks per row
     constexpr int kRowsPerInstr = 32 / kChunksPerRow;                  // rows one warp-wide copy covers
-    // rows of a 128-token tile are dealt to the fifteen gather warps in contiguous runs of 2 x 12 + 13 x 8;
-    // a lane keeps the token id of run row `lane` (and of `lane + 32` for runs longer than a warp)
-    const int row0 = (gw < 2) ? gw * 12 : 24 + (gw - 2) * 8, nrows = (gw < 2) ? 12 : 8;
+    // rows of a 128-token tile are dealt to the seven gather warps in contiguous runs of 4 x 20 + 3 x 16; a lane
+    // keeps the token id of run row `lane`
+    const int row0 = (gw < 4) ? gw * 20 : 80 + (gw - 4) * 16, nrows = (gw < 4) ? 20 : 16;
     const int sub = lane / kChunksPerRow, ch = lane % kChunksPerRow;
     int idx = 0;
     bool ok = true;
     int pending_stage = -1;                                            // tile whose copies are in flight
-    int tokA[2] = {0, 0}, tokB[2] = {0, 0};                            // token ids of the slot's current step
+    int tok0 = 0, tok1 = 0;                                            // token ids of the slots' current steps
     auto load_tokens = [&](int t, int j) {
-      const int pa = j * 128 + row0 + lane, pb = pa + 32;
-      int a = (pa < cnt[t]) ? lst[t][pa] : 0;
-      int b = (lane + 32 < nrows && pb < cnt[t]) ? lst[t][pb] : 0;
+      const int pos = j * 128 + row0 + lane;
+      int a = (lane < nrows && pos < (t ? cnt1 : cnt0)) ? lst[(t ? p.mask_stride : 0) + pos] : 0;
       if (a < 0 || a >= p.S_kv) a = 0;                                    // masked column: any finite row will do
-      if (b < 0 || b >= p.S_kv) b = 0;
-      tokA[t] = a;
-      tokB[t] = b;
+      if (t) tok1 = a;
+      else tok0 = a;
     };
     // Each copy instruction moves whole rows: 16 (D = 128) or 8 (D = 64) neighbouring lanes fetch the
     // consecutive 16-byte chunks of one row, so a warp-wide copy asks L2 for full 128-byte lines
@@ -246,8 +161,7 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
       const __nv_bfloat16* src0 = base + size_t(bh) * p.S_kv * D + ch * 8;
       for (int r = 0; r < nrows; r += kRowsPerInstr) {                 // nrows is a multiple of 4
         const int lr = r + sub;                                        // run row of this lane
-        const int ta = __shfl_sync(0xffffffffu, tokA[t], lr & 31), tb = __shfl_sync(0xffffffffu, tokB[t], lr & 31);
-        const int tok = (lr < 32) ? ta : tb;
+        const int tok = __shfl_sync(0xffffffffu, t ? tok1 : tok0, lr);
         cp_async_16(dst + sw128_offset(row0 + lr, ch & 7), src0 + size_t(tok) * D);
       }
       cp_async_commit();
@@ -260,13 +174,15 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
       ++idx;
     };
     // order: K(0,0) K(1,0), then per step V(t,j) K(t,j+1); the ids of step j serve K(t,j) and V(t,j)
-    if (nst[0] > 0) { load_tokens(0, 0); gather_tile(p.k, 0); }
-    if (nst[1] > 0 && ok) { load_tokens(1, 0); gather_tile(p.k, 1); }
+    if (nst0 > 0) { load_tokens(0, 0); gather_tile(p.k, 0); }
+    if (nst1 > 0 && ok) { load_tokens(1, 0); gather_tile(p.k, 1); }
     for (int j = 0; j < n_max && ok; ++j) {
-      for (int t = 0; t < 2 && ok; ++t) {
-        if (j < nst[t]) {
+#pragma unroll
+      for (int t = 0; t < 2; ++t) {
+        const int n = t ? nst1 : nst0;
+        if (ok && j < n) {
           gather_tile(p.v, t);
-          if (ok && j + 1 < nst[t]) {
+          if (ok && j + 1 < n) {
             load_tokens(t, j + 1);
             gather_tile(p.k, t);
           }
@@ -281,7 +197,7 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
     if (!ok && warp == 8 && lane == 0) mbar_wait_brief(bar(TB_Q_FULL), 0);
   } else if (warp == 9) {
     // ------------------------------------------------------------------ UMMA issuer
-    reg_dealloc<40>();
+    reg_dealloc<48>();
     {   // whole warp, uniform control flow; single instructions go through an elected lane
       const uint32_t idesc_qk = umma_idesc_bf16(128, 128, false);
       const uint32_t idesc_pv = umma_idesc_bf16(128, D, true);
@@ -323,14 +239,15 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
         __syncwarp();
         ++idx;
       };
-      if (ok && nst[0] > 0) qk(0);
-      if (ok && nst[1] > 0) qk(1);
+      if (ok && nst0 > 0) qk(0);
+      if (ok && nst1 > 0) qk(1);
       for (int j = 0; j < n_max && ok; ++j) {
         for (int t = 0; t < 2 && ok; ++t) {
-          if (j < nst[t]) {
+          const int n = t ? nst1 : nst0;
+          if (j < n) {
             pv(t, j);
             if (!ok) break;
-            if (j + 1 < nst[t]) qk(t);
+            if (j + 1 < n) qk(t);
             else umma_commit_elect(bar(TB_O_FULL + t));
           }
         }
@@ -338,7 +255,7 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
     }
   } else {
     // ------------------------------------------------------------------ softmax warpgroups
-    reg_alloc<152>();
+    reg_alloc<208>();
     const int t = warp >> 2, wq = warp & 3;
     const int row = q0 + t * 128 + wq * 32 + lane;
     const uint32_t lane_base = tmem + (uint32_t(wq * 32) << 16);
@@ -346,32 +263,36 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
     OnlineState st;
     online_init(st);
     bool ok = true;
-    // which of a step's 128 gathered columns are real keys; fetched one step ahead so that the list
-    // loads overlap the products of the current step instead of opening every step with a global-memory
-    // round trip
-    uint32_t live[4];
-    auto fetch_live = [&](int j) {
+    // Which of a step's 128 gathered columns are real keys: the entries are requested when the step before has been
+    // computed and looked at when the step's scores are there.
+    const int n_mine = t ? nst1 : nst0, c_mine = t ? cnt1 : cnt0;
+    const int* const l_mine = lst + (t ? p.mask_stride : 0) + lane;
+    int ahead[4];
+    auto request = [&](int j) {
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
-        const int pos = j * 128 + w * 32 + lane;
-        const int tok = (j < nst[t] && pos < cnt[t]) ? lst[t][pos] : -1;
-        live[w] = __ballot_sync(0xffffffffu, tok >= 0 && tok < p.S_kv);
+        const int pos = j * 128 + w * 32;
+        ahead[w] = (pos + lane < c_mine) ? l_mine[pos] : -1;
       }
     };
-    fetch_live(0);
-    for (int j = 0; j < nst[t]; ++j) {
+    request(0);
+    for (int j = 0; j < n_mine; ++j) {
       ok = mbar_wait(bar(TB_S_FULL + t), j & 1, ab, p.err, 901);
       if (!ok) break;
       tc_fence_after();
-      softmax_online_quarters<D>(s_addr, o_addr, p.scale_log2, j == 0, st, live);
+      uint32_t live[4];
+#pragma unroll
+      for (int w = 0; w < 4; ++w) live[w] = __ballot_sync(0xffffffffu, ahead[w] >= 0 && ahead[w] < p.S_kv);
+      float mx0, mx1;
+      softmax_online_step<D, true, 0>(s_addr, s_addr, o_addr, 64, 64, p.scale_log2, j == 0, st, mx0, mx1, live);
       tc_fence_before();
       mbar_arrive(bar(TB_P_FULL + t));
-      fetch_live(j + 1);
+      request(j + 1);
     }
     __nv_bfloat16* orow = p.o + (size_t(bh) * p.S + row) * D;
-    if (skip[t]) {
+    if (t ? skip[1] : skip[0]) {
       // another kernel owns these rows
-    } else if (nst[t] == 0) {
+    } else if (n_mine == 0) {
       if (row < p.S) {
 #pragma unroll
         for (int i = 0; i < D / 8; ++i) reinterpret_cast<uint4*>(orow)[i] = make_uint4(0, 0, 0, 0);
