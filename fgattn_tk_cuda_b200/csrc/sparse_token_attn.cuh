@@ -38,7 +38,7 @@ struct TokenCfg {
   // the products, so the registers go to the softmax warps (208), which hold a row's 128 scores and read them from tensor
   // memory once.  With fifteen gather warps the softmax had 152 and read them twice, 32 at a time: 12 heads of 32760 rows,
   // D = 128, 3276 keys of every block 0.896 -> 0.752 ms, threshold lists (1626 on average) 0.474 -> 0.414; D = 64 0.757 ->
-  // 0.724 and 0.402 -> 0.378 (both with the list entries requested ahead, see the softmax warps).
+  // 0.724 and 0.402 -> 0.378.
   static constexpr int kGatherWarps = 7;
   static constexpr int kGatherThreads = 32 * kGatherWarps;
   static constexpr int kThreads = 32 * (8 + 1 + kGatherWarps);   // 8 softmax warps, the UMMA issuer, the gather warps
@@ -142,14 +142,27 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
     int idx = 0;
     bool ok = true;
     int pending_stage = -1;                                            // tile whose copies are in flight
-    int tok0 = 0, tok1 = 0;                                            // token ids of the slots' current steps
-    auto load_tokens = [&](int t, int j) {
+    // Token ids of the slots' current steps, and the entries of the steps after them, requested a step ahead: asked for when
+    // their tile is next, they held up that tile and the signal of the one before it (3276 keys of 32760, 12 heads, D = 128
+    // 0.752 -> 0.710 ms, D = 64 0.724 -> 0.639; threshold lists 0.414 -> 0.405 and 0.378 -> 0.348).  The copies' own
+    // asynchronous arrival on the stage barriers instead of the wait for the tile before: level; an UMMA issuer per slot
+    // (and six gather warps): 4-13 % slower.
+    int tok0 = 0, tok1 = 0, next0 = 0, next1 = 0;
+    auto request = [&](int t, int j) {
       const int pos = j * 128 + row0 + lane;
-      int a = (lane < nrows && pos < (t ? cnt1 : cnt0)) ? lst[(t ? p.mask_stride : 0) + pos] : 0;
-      if (a < 0 || a >= p.S_kv) a = 0;                                    // masked column: any finite row will do
-      if (t) tok1 = a;
-      else tok0 = a;
+      const int a = (lane < nrows && pos < (t ? cnt1 : cnt0)) ? lst[(t ? p.mask_stride : 0) + pos] : 0;
+      if (t) next1 = a;
+      else next0 = a;
     };
+    auto take_tokens = [&](int t, int j) {                                 // j: the step taken
+      const int a = t ? next1 : next0;
+      const int tok = (a < 0 || a >= p.S_kv) ? 0 : a;                      // masked column: any finite row will do
+      if (t) tok1 = tok;
+      else tok0 = tok;
+      request(t, j + 1);
+    };
+    request(0, 0);
+    request(1, 0);
     // Each copy instruction moves whole rows: 16 (D = 128) or 8 (D = 64) neighbouring lanes fetch the
     // consecutive 16-byte chunks of one row, so a warp-wide copy asks L2 for full 128-byte lines
     // instead of 32 separate sectors.
@@ -174,8 +187,8 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
       ++idx;
     };
     // order: K(0,0) K(1,0), then per step V(t,j) K(t,j+1); the ids of step j serve K(t,j) and V(t,j)
-    if (nst0 > 0) { load_tokens(0, 0); gather_tile(p.k, 0); }
-    if (nst1 > 0 && ok) { load_tokens(1, 0); gather_tile(p.k, 1); }
+    if (nst0 > 0) { take_tokens(0, 0); gather_tile(p.k, 0); }
+    if (nst1 > 0 && ok) { take_tokens(1, 0); gather_tile(p.k, 1); }
     for (int j = 0; j < n_max && ok; ++j) {
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
@@ -183,7 +196,7 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
         if (ok && j < n) {
           gather_tile(p.v, t);
           if (ok && j + 1 < n) {
-            load_tokens(t, j + 1);
+            take_tokens(t, j + 1);
             gather_tile(p.k, t);
           }
         }
