@@ -39,6 +39,8 @@ PROTOTYPES = {
     "fgattn_booleanmask_to_indexmask": (_i, [_vp, _vp, _vp, _i, _i, _i, _i, _i, _vp]),
     "fgattn_all_index_mask": (_i, [_vp, _vp, _i, _i, _i, _i, _i, _vp]),
     "fgattn_sp_attn": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _f, _vp, _sz, _vp]),
+    "fgattn_sp_attn_packed_workspace_bytes": (_sz, [_i, _i, _i, _i]),
+    "fgattn_sp_attn_packed": (_i, [_vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _sz, _vp]),
     "fgattn_block_scratch_bytes": (_sz, [_i, _i, _i, _i]),
     "fgattn_block_index_lists": (_i, [_vp, _vp, _i, _vp, _vp, _vp, _vp, _vp, _vp, _f, _i, _i, _i, _i, _i, _i, _f, _vp,
                                       _sz, _vp]),
@@ -54,6 +56,7 @@ PROTOTYPES = {
     "fgattn_selftest_bounded_wait": (_i, [_ll, _vp]),
     "fgattn_sp_attn_blocks": (_i, [_vp, _vp, _vp, _vp, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _sz, _vp]),
     "fgattn_topk_scratch_bytes": (_sz, [_i, _i, _i, _i, _i, _i]),
+    "fgattn_topk_packed": (_i, [_vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _sz, _vp]),
     "fgattn_topk_indices": (_i, [_vp, _vp, _i, _vp, _vp, _i, _i, _i, _i, _i, _i, _i, _i, _f, _vp, _sz, _vp]),
     "fgattn_pack_mask": (_i, [_vp, _vp, _i, _ll, _i, _vp]),
     "fgattn_unpack_mask": (_i, [_vp, _i, _vp, _ll, _i, _vp]),

@@ -167,6 +167,29 @@ void sp_attn(torch::Tensor o, torch::Tensor q, torch::Tensor k, torch::Tensor v,
                "sp_attn");
 }
 
+// sp_attn on a packed mask instead of lists: uint8 [B,H,ceil(S/128),W/8], one bit per key, of which the first n_valid count.
+// The workspace holds the kept keys of every pair of query blocks, half of what lists would take; it is not kept.
+void sp_attn_packed_check(torch::Tensor o, torch::Tensor q, torch::Tensor k, torch::Tensor v, torch::Tensor packed,
+                          int64_t n_valid) {
+  check_qk(q, k); check_v(v, k); check_o(o, q);
+  check_dtype(packed, at::kByte, "packed");
+  TORCH_CHECK(packed.dim() == 4 && packed.size(0) == q.size(0) && packed.size(1) == q.size(1) &&
+                  packed.size(2) == cdiv(q.size(2), 128) && packed.size(3) >= 1,
+              "packed must be [B, H, ceil(S/128), bytes]");
+  TORCH_CHECK(n_valid >= 0, "n_valid must not be negative");
+}
+void sp_attn_packed(torch::Tensor o, torch::Tensor q, torch::Tensor k, torch::Tensor v, torch::Tensor packed,
+                    int64_t n_valid) {
+  sp_attn_packed_check(o, q, k, v, packed, n_valid);
+  c10::cuda::CUDAGuard guard(q.device());
+  const int64_t bytes = int64_t(fgattn_sp_attn_packed_workspace_bytes(q.size(0), q.size(1), q.size(2), k.size(2)));
+  torch::Tensor ws = torch::empty({bytes}, torch::TensorOptions().dtype(torch::kUInt8).device(q.device()));
+  check_status(fgattn_sp_attn_packed(o.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), packed.data_ptr<uint8_t>(),
+                                     int(packed.size(3)), int(std::min<int64_t>(n_valid, k.size(2))), q.size(0), q.size(1),
+                                     q.size(2), q.size(3), k.size(2), 0.f, ws.data_ptr(), size_t(bytes), stream_of(q)),
+               "sp_attn_packed");
+}
+
 void fullattn_maxq_denom_check(torch::Tensor o, torch::Tensor o_max_q, torch::Tensor o_denom, torch::Tensor q,
                                torch::Tensor k, torch::Tensor v) {
   check_qk(q, k); check_v(v, k); check_o(o, q);
@@ -495,6 +518,26 @@ void topk_indices(torch::Tensor kv_indices, torch::Tensor kv_num_indices, torch:
                                    stream_of(q)), "topk_indices");
 }
 
+// the same selection as bits: uint8 [B,H,ceil(S/blocksz),W/8], W a multiple of 32, one bit per key
+void topk_packed_check(torch::Tensor packed, torch::Tensor q, torch::Tensor k, int64_t select_k, int64_t blocksz) {
+  check_qk(q, k);
+  check_dtype(packed, at::kByte, "packed");
+  TORCH_CHECK(blocksz >= 1 && select_k >= 1 && select_k <= k.size(2), "select_k must lie in [1, S_kv]");
+  TORCH_CHECK(packed.dim() == 4 && packed.size(0) == q.size(0) && packed.size(1) == q.size(1) &&
+                  packed.size(2) == cdiv(q.size(2), blocksz) && packed.size(3) % 4 == 0 && packed.size(3) * 8 >= k.size(2),
+              "packed must be [B, H, ceil(S/blocksz), >= S_kv / 8, a multiple of 4]");
+}
+void topk_packed(torch::Tensor packed, torch::Tensor q, torch::Tensor k, int64_t select_k, int64_t blocksz) {
+  topk_packed_check(packed, q, k, select_k, blocksz);
+  c10::cuda::CUDAGuard guard(q.device());
+  const int64_t bytes = int64_t(fgattn_topk_scratch_bytes(q.size(0), q.size(1), q.size(2), q.size(3), int(blocksz),
+                                                          int(k.size(2))));
+  torch::Tensor scratch = torch::empty({bytes}, torch::TensorOptions().dtype(torch::kUInt8).device(q.device()));
+  check_status(fgattn_topk_packed(packed.data_ptr<uint8_t>(), int(packed.size(3)), q.data_ptr(), k.data_ptr(), int(select_k),
+                                  q.size(0), q.size(1), q.size(2), q.size(3), int(blocksz), k.size(2), k.size(2), 0.f,
+                                  scratch.data_ptr(), size_t(bytes), stream_of(q)), "topk_packed");
+}
+
 int64_t block_scratch_bytes(int64_t batch, int64_t heads, int64_t seq, int64_t kv_seq_len) {
   return int64_t(fgattn_block_scratch_bytes(int(batch), int(heads), int(seq), int(kv_seq_len)));
 }
@@ -514,6 +557,7 @@ TORCH_LIBRARY_FRAGMENT(cuda_attn, m) {
   m.def("booleanmask_128_listed(Tensor (booleanmask!) booleanmask, Tensor o_max_q, Tensor o_denom, Tensor q, Tensor k, float threshold, Tensor kb_indices, Tensor kb_counts) -> ()");
   m.def("packedmask_128_listed(Tensor (packed!) packed, Tensor o_max_q, Tensor o_denom, Tensor q, Tensor k, float threshold, Tensor kb_indices, Tensor kb_counts) -> ()");
   m.def("packedmask_to_lists(Tensor (indices!) indices, Tensor (num_indices!) num_indices, Tensor packed, int n_valid) -> ()");
+  m.def("sp_attn_packed(Tensor (o!) o, Tensor q, Tensor k, Tensor v, Tensor packed, int n_valid) -> ()");
   m.def("block_index_lists(Tensor (kb_indices!) kb_indices, Tensor (kb_counts!) kb_counts, Tensor (o_max_q!) o_max_q, Tensor (o_denom!) o_denom, Tensor(o!)? o, Tensor q, Tensor k, Tensor? v, float threshold, Tensor (scratch!) scratch) -> ()");
   m.def("block_lists_from_maxima(Tensor (kb_indices!) kb_indices, Tensor (kb_counts!) kb_counts, Tensor block_maxima, Tensor max_q, Tensor denom, int seq, int head_dim, int kv_seq_len, float threshold) -> ()");
   m.def("sp_attn_blocks_ml(Tensor (o!) o, Tensor q, Tensor k, Tensor v, Tensor kb_indices, Tensor kb_counts, Tensor max_q, Tensor denom) -> ()");
@@ -526,6 +570,7 @@ TORCH_LIBRARY_FRAGMENT(cuda_attn, m) {
   m.def("indexmask_to_packedmask(Tensor (packed!) packed, Tensor indices, Tensor num_indices) -> ()");
   // top-k selector
   m.def("topk_indices(Tensor (kv_indices!) kv_indices, Tensor (kv_num_indices!) kv_num_indices, Tensor q, Tensor k, int select_k, int blocksz) -> ()");
+  m.def("topk_packed(Tensor (packed!) packed, Tensor q, Tensor k, int select_k, int blocksz) -> ()");
 }
 
 // Meta kernels: every operator writes into caller-allocated tensors and returns nothing, so the Meta
@@ -541,6 +586,7 @@ TORCH_LIBRARY_IMPL(cuda_attn, Meta, m) {
   m.impl("booleanmask_128_listed", booleanmask_128_listed_check);
   m.impl("packedmask_128_listed", packedmask_128_listed_check);
   m.impl("packedmask_to_lists", packedmask_to_lists_check);
+  m.impl("sp_attn_packed", sp_attn_packed_check);
   m.impl("block_index_lists", block_index_lists_check);
   m.impl("block_lists_from_maxima", block_lists_from_maxima_check);
   m.impl("sp_attn_blocks_ml", sp_attn_blocks_ml_check);
@@ -551,6 +597,7 @@ TORCH_LIBRARY_IMPL(cuda_attn, Meta, m) {
   m.impl("packedmask_to_indexmask", packedmask_to_indexmask_check);
   m.impl("indexmask_to_packedmask", indexmask_to_packedmask_check);
   m.impl("topk_indices", topk_indices_check);
+  m.impl("topk_packed", topk_packed_check);
 }
 
 TORCH_LIBRARY_IMPL(cuda_attn, CUDA, m) {
@@ -564,6 +611,7 @@ TORCH_LIBRARY_IMPL(cuda_attn, CUDA, m) {
   m.impl("booleanmask_128_listed", booleanmask_128_listed);
   m.impl("packedmask_128_listed", packedmask_128_listed);
   m.impl("packedmask_to_lists", packedmask_to_lists);
+  m.impl("sp_attn_packed", sp_attn_packed);
   m.impl("block_index_lists", block_index_lists);
   m.impl("block_lists_from_maxima", block_lists_from_maxima);
   m.impl("sp_attn_blocks_ml", sp_attn_blocks_ml);
@@ -574,6 +622,7 @@ TORCH_LIBRARY_IMPL(cuda_attn, CUDA, m) {
   m.impl("packedmask_to_indexmask", packedmask_to_indexmask);
   m.impl("indexmask_to_packedmask", indexmask_to_packedmask);
   m.impl("topk_indices", topk_indices);
+  m.impl("topk_packed", topk_packed);
 }
 
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {

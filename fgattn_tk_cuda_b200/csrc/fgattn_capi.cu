@@ -549,6 +549,76 @@ int fgattn_all_index_mask(int* kv_indices, int* kv_num_indices, int batch, int h
   return FGATTN_OK;
 }
 
+namespace {
+// What every form of the token-list attention sets up: sizes, tensors and maps.
+int token_setup(fg::TokenParams& p, CUtensorMap& mq, CUtensorMap& mo, void* o, const void* q, const void* k, const void* v,
+                int batch, int heads, int seq, int D, int kv_rows, float scale) {
+  memset(&p, 0, sizeof(p));
+  p.o = static_cast<__nv_bfloat16*>(o);
+  p.k = static_cast<const __nv_bfloat16*>(k);
+  p.v = static_cast<const __nv_bfloat16*>(v);
+  p.S = seq;
+  p.S_kv = kv_rows;
+  p.nqb = (seq + 127) / 128;
+  p.scale_log2 = resolve_scale_log2(scale, D);
+  int r = get_err_word(&p.err);
+  if (r) return r;
+  if (fg::make_qkv_map(&mq, q, batch * heads, seq, D, 128) || fg::make_qkv_map(&mo, o, batch * heads, seq, D, 32))
+    return fg::encode_tiled_fn() ? FGATTN_INVALID_ARGUMENT : FGATTN_NO_DRIVER;
+  p.pairs = (seq + 255) / 256;
+  if ((long long)batch * heads * p.pairs > 2147483647LL) return FGATTN_UNSUPPORTED;
+  return FGATTN_OK;
+}
+
+// The order of the thread blocks (len[item * subs + j], j < subs, of len_rows per unit: what item is long by) and the kernel.
+int token_launch(fg::TokenParams& p, const CUtensorMap& mq, const CUtensorMap& mo, int n_units, int D, int kv_rows,
+                 void* workspace, const int* len, int len_rows, int subs, int shift, cudaStream_t st) {
+  int sms = 0;
+  int r = sm_count(&sms);
+  if (r) return r;
+  if (workspace && n_units * p.pairs > sms) {       // (no order for fewer items than SMs)
+    // thread-block order: inside groups of units, longest lists first.  The row gather gains little from
+    // L2 residency of K/V, and large groups balance better (measured at (1,12,32760,128): 0.90 ms in
+    // storage order, 0.77 ms with 4 heads per group, 0.55 ms with all 12), so groups span up to 256 MiB of K/V.
+    const size_t kv_bytes_per_unit = size_t(4) * kv_rows * D;
+    int group = int(std::max<size_t>(1, (size_t(256) << 20) / kv_bytes_per_unit));
+    if (env_group_heads() > 0) group = env_group_heads();                // tuning override
+    group = std::max(1, std::min(group, n_units));
+    const int n_groups = (n_units + group - 1) / group;
+    group = (n_units + n_groups - 1) / n_groups;                      // groups of equal size
+    int* ws = static_cast<int*>(workspace);
+    fg::sparse_order_kernel<<<(n_units + group - 1) / group, 1024, 0, st>>>(len, ws + 4, ws, len_rows, p.pairs, n_units,
+                                                                          group, subs, 1, shift);
+    FG_CUDA(cudaGetLastError());
+    p.order = ws + 4;
+  }
+  dim3 grid(n_units * p.pairs, 1, 1);
+  if (D == 128) {
+    auto kern = fg::sparse_token_attn_kernel<128>;
+    r = set_smem(kern, fg::TokenCfg<128>::kSmemBytes);
+    if (r) return r;
+    kern<<<grid, fg::TokenCfg<128>::kThreads, fg::TokenCfg<128>::kSmemBytes, st>>>(mq, mo, p);
+  } else {
+    auto kern = fg::sparse_token_attn_kernel<64>;
+    r = set_smem(kern, fg::TokenCfg<64>::kSmemBytes);
+    if (r) return r;
+    kern<<<grid, fg::TokenCfg<64>::kThreads, fg::TokenCfg<64>::kSmemBytes, st>>>(mq, mo, p);
+  }
+  FG_CUDA(cudaGetLastError());
+  return FGATTN_OK;
+}
+
+// Keys of one pair of query blocks: every key once and less than a tile of common ones twice.
+int packed_pair_cap(int kv_rows) { return kv_rows + 128; }
+}  // namespace
+
+size_t fgattn_sp_attn_packed_workspace_bytes(int batch, int heads, int seq, int kv_rows) {
+  if (batch <= 0 || heads <= 0 || seq <= 0 || kv_rows <= 0) return 0;
+  const size_t n_pairs = size_t(batch) * heads * ((seq + 255) / 256);
+  return align256(fgattn_sp_attn_workspace_bytes(batch, heads, seq)) + align256(n_pairs * sizeof(int4)) +
+         align256(n_pairs * sizeof(int)) + align256(n_pairs * packed_pair_cap(kv_rows) * sizeof(int));
+}
+
 int fgattn_sp_attn(void* o, const void* q, const void* k, const void* v, const int* kv_indices,
                    const int* kv_num_indices, int mask_stride, int batch, int heads, int seq, int D, int kv_rows,
                    float scale, void* workspace, size_t workspace_bytes, void* stream) {
@@ -559,26 +629,14 @@ int fgattn_sp_attn(void* o, const void* q, const void* k, const void* v, const i
   if (workspace && !aligned16(workspace)) return FGATTN_MISALIGNED;
   if (workspace && workspace_bytes < fgattn_sp_attn_workspace_bytes(batch, heads, seq)) return FGATTN_SCRATCH_TOO_SMALL;
   fg::TokenParams p;
-  memset(&p, 0, sizeof(p));
-  p.o = static_cast<__nv_bfloat16*>(o);
-  p.k = static_cast<const __nv_bfloat16*>(k);
-  p.v = static_cast<const __nv_bfloat16*>(v);
+  CUtensorMap mq, mo;
+  r = token_setup(p, mq, mo, o, q, k, v, batch, heads, seq, D, kv_rows, scale);
+  if (r) return r;
   p.kv_idx = kv_indices;
   p.kv_cnt = kv_num_indices;
-  p.S = seq;
-  p.S_kv = kv_rows;
-  p.nqb = (seq + 127) / 128;
   p.mask_stride = mask_stride;
-  p.scale_log2 = resolve_scale_log2(scale, D);
-  r = get_err_word(&p.err);
-  if (r) return r;
-  CUtensorMap mq, mo;
-  if (fg::make_qkv_map(&mq, q, batch * heads, seq, D, 128) || fg::make_qkv_map(&mo, o, batch * heads, seq, D, 32))
-    return fg::encode_tiled_fn() ? FGATTN_INVALID_ARGUMENT : FGATTN_NO_DRIVER;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  p.pairs = (seq + 255) / 256;
   const int n_units = batch * heads;
-  if ((long long)n_units * p.pairs > 2147483647LL) return FGATTN_UNSUPPORTED;
   // ---- block route: with the large workspace, query blocks whose lists nearly fill the 64-key blocks they
   // touch are computed from whole K/V tiles (TMA by block index, unlisted columns switched off) on the
   // persistent fixed-offset kernel; the others stay on the row gather below
@@ -630,41 +688,39 @@ int fgattn_sp_attn(void* o, const void* q, const void* k, const void* v, const i
     if (r) return r;
     p.route = route;
   }
-  int sms = 0;
-  r = sm_count(&sms);
+  int shift = 0;
+  while ((mask_stride >> shift) >= 1024) ++shift;                     // bucketed list lengths
+  return token_launch(p, mq, mo, n_units, D, kv_rows, workspace, kv_num_indices, p.nqb, 2, shift, st);
+}
+
+int fgattn_sp_attn_packed(void* o, const void* q, const void* k, const void* v, const unsigned char* packed, int row_bytes,
+                          int n_valid, int batch, int heads, int seq, int D, int kv_rows, float scale, void* workspace,
+                          size_t workspace_bytes, void* stream) {
+  int r = check_qk(q, k, batch, heads, seq, D, kv_rows, kv_rows);
   if (r) return r;
-  if (workspace && n_units * p.pairs > sms) {       // (no order for fewer items than SMs)
-    // thread-block order: inside groups of units, longest lists first.  The row gather gains little from
-    // L2 residency of K/V, and large groups balance better (measured at (1,12,32760,128): 0.90 ms in
-    // storage order, 0.77 ms with 4 heads per group, 0.55 ms with all 12), so groups span up to 256 MiB of K/V.
-    const size_t kv_bytes_per_unit = size_t(4) * kv_rows * D;
-    int group = int(std::max<size_t>(1, (size_t(256) << 20) / kv_bytes_per_unit));
-    if (env_group_heads() > 0) group = env_group_heads();                // tuning override
-    group = std::max(1, std::min(group, n_units));
-    const int n_groups = (n_units + group - 1) / group;
-    group = (n_units + n_groups - 1) / n_groups;                      // groups of equal size
-    int shift = 0;
-    while ((mask_stride >> shift) >= 1024) ++shift;                   // bucketed list lengths
-    int* ws = static_cast<int*>(workspace);
-    fg::sparse_order_kernel<<<(n_units + group - 1) / group, 1024, 0, st>>>(kv_num_indices, ws + 4, ws, p.nqb, p.pairs,
-                                                                          n_units, group, 2, 1, shift);
-    FG_CUDA(cudaGetLastError());
-    p.order = ws + 4;
-  }
-  dim3 grid(n_units * p.pairs, 1, 1);
-  if (D == 128) {
-    auto kern = fg::sparse_token_attn_kernel<128>;
-    r = set_smem(kern, fg::TokenCfg<128>::kSmemBytes);
-    if (r) return r;
-    kern<<<grid, fg::TokenCfg<128>::kThreads, fg::TokenCfg<128>::kSmemBytes, st>>>(mq, mo, p);
-  } else {
-    auto kern = fg::sparse_token_attn_kernel<64>;
-    r = set_smem(kern, fg::TokenCfg<64>::kSmemBytes);
-    if (r) return r;
-    kern<<<grid, fg::TokenCfg<64>::kThreads, fg::TokenCfg<64>::kSmemBytes, st>>>(mq, mo, p);
-  }
+  if (!o || !v || !packed || !workspace || row_bytes < 1 || n_valid < 0) return FGATTN_INVALID_ARGUMENT;
+  if (kv_rows >= (1 << 21)) return FGATTN_UNSUPPORTED;     // counts of 21 bits (packed_pairs_kernel)
+  if (!aligned16(o) || !aligned16(v) || !aligned16(workspace)) return FGATTN_MISALIGNED;
+  if (workspace_bytes < fgattn_sp_attn_packed_workspace_bytes(batch, heads, seq, kv_rows)) return FGATTN_SCRATCH_TOO_SMALL;
+  fg::TokenParams p;
+  CUtensorMap mq, mo;
+  r = token_setup(p, mq, mo, o, q, k, v, batch, heads, seq, D, kv_rows, scale);
+  if (r) return r;
+  cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const int n_units = batch * heads;
+  const size_t n_pairs = size_t(n_units) * p.pairs;
+  char* base = static_cast<char*>(workspace) + align256(fgattn_sp_attn_workspace_bytes(batch, heads, seq));
+  int4* split = reinterpret_cast<int4*>(base);
+  int* cost = reinterpret_cast<int*>(base + align256(n_pairs * sizeof(int4)));
+  int* lists = reinterpret_cast<int*>(base + align256(n_pairs * sizeof(int4)) + align256(n_pairs * sizeof(int)));
+  p.split = split;
+  p.pair_lists = lists;
+  p.pair_cap = packed_pair_cap(kv_rows);
+  fg::packed_pairs_kernel<<<dim3(p.pairs, n_units), 256, 0, st>>>(
+      packed, row_bytes, int(std::min<long long>(std::min(n_valid, kv_rows), 8LL * row_bytes)), p.nqb, p.pairs, p.pair_cap,
+      lists, split, cost);
   FG_CUDA(cudaGetLastError());
-  return FGATTN_OK;
+  return token_launch(p, mq, mo, n_units, D, kv_rows, workspace, cost, p.pairs, 1, 0, st);
 }
 
 size_t fgattn_sp_attn_token_workspace_bytes(int batch, int heads, int seq, int kv_rows) {
@@ -1037,13 +1093,16 @@ size_t fgattn_topk_scratch_bytes(int batch, int heads, int seq, int D, int block
   return 2 * align256(bh * nblk * D * 2) + bh * nblk * s_stride * sizeof(float);
 }
 
-int fgattn_topk_indices(int* kv_indices, int* kv_num_indices, int list_stride, const void* q, const void* k,
+namespace {
+// Either lists (kv_indices, kv_num_indices, list_stride) or bits (rows of row_bytes).
+int topk_select(int* kv_indices, int* kv_num_indices, int list_stride, uint32_t* bits, int row_bytes, const void* q, const void* k,
                         int select_k, int batch, int heads, int seq, int D, int blocksz, int kv_rows, int kv_seq_len,
                         float scale, void* scratch, size_t scratch_bytes, void* stream) {
   int r = check_qk(q, k, batch, heads, seq, D, kv_rows, kv_seq_len);
   if (r) return r;
-  if (!kv_indices || !kv_num_indices || !scratch || blocksz < 1) return FGATTN_INVALID_ARGUMENT;
-  if (select_k < 1 || select_k > kv_seq_len || list_stride < select_k) return FGATTN_INVALID_ARGUMENT;
+  if ((!bits && (!kv_indices || !kv_num_indices)) || !scratch || blocksz < 1) return FGATTN_INVALID_ARGUMENT;
+  if (select_k < 1 || select_k > kv_seq_len || (!bits && list_stride < select_k)) return FGATTN_INVALID_ARGUMENT;
+  if (bits && (row_bytes % 4 || (long long)row_bytes * 8 < kv_seq_len)) return FGATTN_INVALID_ARGUMENT;
   if (select_k > 8192) return FGATTN_UNSUPPORTED;          // the selected pairs are sorted in shared memory
   if (!aligned16(scratch)) return FGATTN_MISALIGNED;
   if (scratch_bytes < fgattn_topk_scratch_bytes(batch, heads, seq, D, blocksz, kv_seq_len))
@@ -1068,7 +1127,14 @@ int fgattn_topk_indices(int* kv_indices, int* kv_num_indices, int list_stride, c
   if (fg::make_qkv_map(&m_hi, qm_hi, bh, nblk, D, 128) || fg::make_qkv_map(&m_lo, qm_lo, bh, nblk, D, 128) ||
       fg::make_qkv_map(&mk, k, bh, kv_rows, D, 128))
     return fg::encode_tiled_fn() ? FGATTN_INVALID_ARGUMENT : FGATTN_NO_DRIVER;
-  const dim3 g_mean(nblk, bh), g_sc(s_stride / 128, (nblk + 127) / 128, bh);
+  p.k_tiles = s_stride / 128;
+  p.q_tiles = (nblk + 127) / 128;
+  if ((long long)bh * p.q_tiles * p.k_tiles > 2147483647LL) return FGATTN_UNSUPPORTED;
+  p.n_tiles = bh * p.q_tiles * p.k_tiles;
+  int sms = 0;
+  r = sm_count(&sms);
+  if (r) return r;
+  const dim3 g_mean(nblk, bh), g_sc(std::min(p.n_tiles, sms));
   if (D == 128) {
     fg::qblock_mean_kernel<128><<<g_mean, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(q), qm_hi, qm_lo, seq, nblk,
                                                        blocksz, sc);
@@ -1087,13 +1153,35 @@ int fgattn_topk_indices(int* kv_indices, int* kv_num_indices, int list_stride, c
   FG_CUDA(cudaGetLastError());
   int k_pow2 = 2;
   while (k_pow2 < select_k) k_pow2 <<= 1;
-  const int smem_sel = k_pow2 * 10;
-  r = set_smem(fg::topk_select_kernel, std::max(smem_sel, 1024));
-  if (r) return r;
-  fg::topk_select_kernel<<<unsigned(bh * nblk), fg::kSelThreads, smem_sel, st>>>(
-      scores, s_stride, kv_seq_len, select_k, k_pow2, kv_indices, kv_num_indices, list_stride);
-  FG_CUDA(cudaGetLastError());
-  return FGATTN_OK;
+  const int cap = fg::select_capacity(select_k);
+  const int smem_sel = 8 * (cap + int(fg::kSelBinSort)) + (bits ? row_bytes : 2 * cap);
+  if (smem_sel > 200 * 1024) return FGATTN_UNSUPPORTED;    // rows of more than 800000 bits beside the largest selection
+  auto go = [&](auto kern) -> int {
+    int rr = set_smem(kern, smem_sel);
+    if (rr) return rr;
+    kern<<<unsigned(bh * nblk), fg::kSelThreads, smem_sel, st>>>(scores, s_stride, kv_seq_len, select_k, k_pow2, cap, kv_indices,
+                                                               kv_num_indices, list_stride, bits, row_bytes / 4);
+    FG_CUDA(cudaGetLastError());
+    return FGATTN_OK;
+  };
+  return bits ? go(fg::topk_select_kernel<true>) : go(fg::topk_select_kernel<false>);
+}
+}  // namespace
+
+int fgattn_topk_indices(int* kv_indices, int* kv_num_indices, int list_stride, const void* q, const void* k,
+                        int select_k, int batch, int heads, int seq, int D, int blocksz, int kv_rows, int kv_seq_len,
+                        float scale, void* scratch, size_t scratch_bytes, void* stream) {
+  return topk_select(kv_indices, kv_num_indices, list_stride, nullptr, 0, q, k, select_k, batch, heads, seq, D, blocksz,
+                     kv_rows, kv_seq_len, scale, scratch, scratch_bytes, stream);
+}
+
+int fgattn_topk_packed(unsigned char* packed, int row_bytes, const void* q, const void* k, int select_k, int batch, int heads,
+                       int seq, int D, int blocksz, int kv_rows, int kv_seq_len, float scale, void* scratch,
+                       size_t scratch_bytes, void* stream) {
+  if (!packed) return FGATTN_INVALID_ARGUMENT;
+  if (reinterpret_cast<uintptr_t>(packed) & 3u) return FGATTN_MISALIGNED;
+  return topk_select(nullptr, nullptr, 0, reinterpret_cast<uint32_t*>(packed), row_bytes, q, k, select_k, batch, heads, seq, D,
+                     blocksz, kv_rows, kv_seq_len, scale, scratch, scratch_bytes, stream);
 }
 
 }  // extern "C"

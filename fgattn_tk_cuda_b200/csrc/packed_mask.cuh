@@ -59,6 +59,36 @@ unpack_mask_kernel(const uint8_t* __restrict__ packed, T* __restrict__ mask, lon
   }
 }
 
+// The set bits of a warp's 32 words (bits: lane's word, c: how many, at: slot of the first), words first .. first + 31 of a
+// row, as entries of the list dst; slots from limit on are left alone.
+// Two ways to write the warp's entries.  Word by word, a lane per bit: a trip per non-empty word, its entries in one
+// store -- for masks whose bits come in runs.  Or every lane its own word, bit by bit: as many trips as the fullest
+// word has bits, each spread over about as many lines -- for scattered bits, a few in almost every word.
+// 3072 rows of 32768 bits, us by words / by bits: set in runs, 5 % in runs of 256 20 / 37, 15 % in runs of 8 53 / 72;
+// scattered, 1 % 35 / 16, 5 % 78 / 23, 10 % 89 / 31, 20 % 92 / 78, 50 % 93 / 291.  A trip by bits costs the more
+// the more bits the words hold; most^2 / 5 trips by words are where the two meet.
+__device__ __forceinline__ void write_entries(uint32_t bits, int c, int at, int first, int* __restrict__ dst, int limit) {
+  const int lane = threadIdx.x & 31;
+  uint32_t todo = __ballot_sync(0xffffffffu, bits != 0u);
+  const int most = __reduce_max_sync(0xffffffffu, c);
+  if (5 * __popc(todo) <= most * most) {
+    while (todo) {
+      const int from = __ffs(todo) - 1;
+      todo &= todo - 1;
+      const uint32_t u = __shfl_sync(0xffffffffu, bits, from);
+      const int slot = __shfl_sync(0xffffffffu, at, from) + __popc(u & ((1u << lane) - 1u));
+      if (((u >> lane) & 1u) && slot < limit) dst[slot] = 32 * (first + from) + lane;
+    }
+  } else {
+    while (bits) {
+      const int e = __ffs(bits) - 1;
+      bits &= bits - 1;
+      if (at < limit) dst[at] = 32 * (first + lane) + e;
+      ++at;
+    }
+  }
+}
+
 // Packed mask row -> ascending index list + count.  Row r of `packed` has row_bytes bytes; entry e is
 // kept iff its bit is set and e < n_valid.  Unused list slots receive `sentinel`.  grid (rows), 256
 // threads; each thread owns four 32-entry words per sweep.  FILL = false leaves the unused slots as they are: a
@@ -124,32 +154,7 @@ packed_to_index_kernel(const uint8_t* __restrict__ packed, int row_bytes, int* _
         chunk_total += t;
       }
       mine += incl[k] - c[k];
-      // Two ways to write the warp's entries.  Word by word, a lane per bit: a trip per non-empty word, its entries in one
-      // store -- for masks whose bits come in runs.  Or every lane its own word, bit by bit: as many trips as the fullest
-      // word has bits, each spread over about as many lines -- for scattered bits, a few in almost every word.
-      // 3072 rows of 32768 bits, us by words / by bits: set in runs, 5 % in runs of 256 20 / 37, 15 % in runs of 8 53 / 72;
-      // scattered, 1 % 35 / 16, 5 % 78 / 23, 10 % 89 / 31, 20 % 92 / 78, 50 % 93 / 291.  A trip by bits costs the more
-      // the more bits the words hold; most^2 / 5 trips by words are where the two meet.
-      uint32_t todo = __ballot_sync(0xffffffffu, bits[k] != 0u);
-      const int most = __reduce_max_sync(0xffffffffu, c[k]);
-      if (5 * __popc(todo) <= most * most) {
-        while (todo) {
-          const int from = __ffs(todo) - 1;
-          todo &= todo - 1;
-          const uint32_t u = __shfl_sync(0xffffffffu, bits[k], from);
-          const int slot = __shfl_sync(0xffffffffu, mine, from) + __popc(u & ((1u << lane) - 1u));
-          if (((u >> lane) & 1u) && slot < list_stride) dst[slot] = 32 * (w0 + k * 256 + warp * 32 + from) + lane;
-        }
-      } else {
-        const int w = w0 + k * 256 + tid;
-        uint32_t u = bits[k];
-        while (u) {
-          const int e = __ffs(u) - 1;
-          u &= u - 1;
-          if (mine < list_stride) dst[mine] = 32 * w + e;
-          ++mine;
-        }
-      }
+      write_entries(bits[k], c[k], mine, w0 + k * 256 + warp * 32, dst, list_stride);
       off += chunk_total;
     }
     __syncthreads();
@@ -183,6 +188,116 @@ index_to_packed_kernel(const int* __restrict__ idx, const int* __restrict__ cnt,
     for (int w = tid; w < n_words; w += 256) reinterpret_cast<uint32_t*>(dst)[w] = s_bits[w];
   } else {
     for (int b = tid; b < row_bytes; b += 256) dst[b] = uint8_t(s_bits[b >> 2] >> (8 * (b & 3)));
+  }
+}
+
+// Packed masks of two neighbouring query blocks -> what both keep, in whole tiles of 128 keys, and what is left of each.
+//
+// The token-list attention runs two 128-row query blocks per thread block, and what bounds it is the row gather: every
+// kept key's K and V row is fetched once for each of the two.  Neighbouring blocks keep much the same keys (rows of one
+// region of the sequence look at the same part of it), so the tiles of common keys are fetched once for both.  A block's
+// number of 128-key steps is what its own list would take: common keys past the last whole tile go to both remainders.
+// Per pair the list row of `cap` entries holds 128 x common keys, then the remainder of the first block (y keys), then that
+// of the second (z); split = (x, y, z, 0), cost = tiles to gather.  All three ascend.
+// 12 heads of 256 query blocks and 32760 keys, 5 % kept: 36 us, where the lists of all blocks took 45 (packed_to_index_kernel).
+// Entries put together in shared memory first, to leave as whole lines: 36 to 50 us (bank conflicts).  Sharing is worth
+// up to 7 % of the attention there, as long as what bounds a step is the chain of softmax and products: on lists handed
+// over by a program, where finding the common keys is a pass of its own over them, it was level to 12 % slower.
+// grid (pairs, BH), 256 threads, 1024 words of either mask per sweep.  Counts travel three to a 64-bit word.
+__global__ void __launch_bounds__(256, 5)
+packed_pairs_kernel(const uint8_t* __restrict__ packed, int row_bytes, int n_valid, int nqb, int pairs, int cap,
+                    int* __restrict__ lists, int4* __restrict__ split, int* __restrict__ cost) {
+  constexpr int kChunks = 4, kWarps = 8, kSweep = 256 * kChunks;
+  static_assert(kChunks * kWarps == 32, "a lane per chunk and warp");
+  __shared__ unsigned long long part[32];                // [chunk][warp]: common, first alone, second alone, 21 bits each
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int qb = 2 * blockIdx.x;
+  const size_t item = size_t(blockIdx.y) * pairs + blockIdx.x;
+  const uint8_t* src0 = packed + (size_t(blockIdx.y) * nqb + qb) * row_bytes;
+  const bool two = qb + 1 < nqb, words = ((row_bytes & 3) == 0) && ((reinterpret_cast<uintptr_t>(src0) & 3) == 0);
+  const int n_words = min((row_bytes + 3) >> 2, (n_valid + 31) >> 5);
+  auto word_of = [&](const uint8_t* src, int w) -> uint32_t {
+    uint32_t u = 0;
+    if (words) {
+      u = reinterpret_cast<const uint32_t*>(src)[w];
+    } else {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        if (4 * w + e < row_bytes) u |= uint32_t(src[4 * w + e]) << (8 * e);
+    }
+    const int left = n_valid - 32 * w;
+    return left < 32 ? u & ((1u << left) - 1u) : u;      // (left > 0: w < n_words)
+  };
+  auto counts_of = [](uint32_t a, uint32_t b) -> unsigned long long {
+    return (unsigned long long)(__popc(a & b)) | (unsigned long long)(__popc(a & ~b)) << 21 |
+           (unsigned long long)(__popc(b & ~a)) << 42;
+  };
+  auto scan = [&](unsigned long long x) {                // inclusive, over the lanes
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const unsigned long long t = __shfl_up_sync(0xffffffffu, x, o);
+      if (lane >= o) x += t;
+    }
+    return x;
+  };
+  auto field = [](unsigned long long x, int i) { return int(x >> (21 * i)) & 0x1fffff; };
+
+  unsigned long long base = 0, total = 0;                // entries of the sweeps before this one, and of all
+  if (n_words > kSweep) {
+    for (int w = tid; w < n_words; w += 256) total += counts_of(word_of(src0, w), two ? word_of(src0 + row_bytes, w) : 0u);
+    total = scan(total);
+    if (lane == 31) part[warp] = total;
+    __syncthreads();
+    total = 0;
+#pragma unroll
+    for (int w = 0; w < kWarps; ++w) total += part[w];
+    __syncthreads();
+  }
+  int* const out = lists + item * cap;
+  for (int w0 = 0; w0 < n_words || w0 == 0; w0 += kSweep) {
+    uint32_t a[kChunks], b[kChunks];
+    unsigned long long c[kChunks], incl[kChunks];
+#pragma unroll
+    for (int k = 0; k < kChunks; ++k) {
+      const int w = w0 + k * 256 + tid;
+      a[k] = w < n_words ? word_of(src0, w) : 0u;
+      b[k] = (w < n_words && two) ? word_of(src0 + row_bytes, w) : 0u;
+    }
+#pragma unroll
+    for (int k = 0; k < kChunks; ++k) {
+      c[k] = counts_of(a[k], b[k]);
+      incl[k] = scan(c[k]);
+      if (lane == 31) part[k * kWarps + warp] = incl[k];
+    }
+    __syncthreads();
+    const unsigned long long mine = part[lane], upto = scan(mine);
+    const unsigned long long sweep = __shfl_sync(0xffffffffu, upto, 31);
+    if (n_words <= kSweep) total = sweep;
+    const int tiles = field(total, 0) >> 7, whole = tiles << 7, rest = field(total, 0) & 127;
+    const int len0 = rest + field(total, 1), len1 = rest + field(total, 2);
+    int* const out1 = out + whole + len0;                // the second block's remainder
+    if (tid == 0 && w0 == 0) {
+      split[item] = make_int4(tiles, len0, len1, 0);
+      cost[item] = tiles + ((len0 + 127) >> 7) + ((len1 + 127) >> 7);
+    }
+#pragma unroll
+    for (int k = 0; k < kChunks; ++k) {
+      const unsigned long long at = base + __shfl_sync(0xffffffffu, upto - mine, k * kWarps + warp) + incl[k] - c[k];
+      const int first = w0 + k * 256 + warp * 32;
+      const int at0 = field(at, 0);
+      const uint32_t both = a[k] & b[k];
+      // the common keys, of which the last `rest` are where the first remainder starts, and once more in the second
+      write_entries(both, field(c[k], 0), at0, first, out, cap);
+      if (__any_sync(0xffffffffu, at0 + field(c[k], 0) > whole)) {
+        uint32_t u = both;
+        for (int e = at0; u; ++e, u &= u - 1)
+          if (e >= whole) out1[e - whole] = 32 * (first + lane) + __ffs(u) - 1;
+      }
+      write_entries(a[k] & ~b[k], field(c[k], 1), field(at, 1), first, out + field(total, 0), cap);
+      write_entries(b[k] & ~a[k], field(c[k], 2), field(at, 2), first, out1 + rest, cap);
+    }
+    base += sweep;
+    __syncthreads();                                     // `part` is free for the next sweep
   }
 }
 

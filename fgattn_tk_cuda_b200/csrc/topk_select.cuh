@@ -7,12 +7,12 @@
 //   qblock_mean_kernel   : block means of q in fp32, written as a bf16 pair hi + lo (hi = bf16(mean),
 //                          lo = bf16(mean - hi)), so that two bf16 tensor-core products reproduce
 //                          the fp32 mean to ~2^-17 relative.  HBM-bound read of q.
-//   topk_scores_kernel   : scores = (hi + lo) . k^T on tcgen05 (128 query blocks x 128 keys per
-//                          CTA, accumulator in TMEM), staged through shared memory and written as
-//                          fp32 rows; columns past kv_len hold -inf.
-//   topk_select_kernel   : per row an interval-narrowing histogram select (2048 bins per sweep) for
-//                          the k-th largest score, ordered tie handling (smallest key index first),
-//                          then the selected (score, index) pairs put in order in shared memory.
+//   topk_scores_kernel   : scores = (hi + lo) . k^T on tcgen05 (tiles of 128 query blocks x 128 keys,
+//                          accumulators in TMEM), written as fp32 rows; columns past kv_len hold -inf.
+//   topk_select_kernel   : per row a threshold from a sample and one sweep that collects, or an interval-narrowing
+//                          histogram select (2048 bins per sweep) for the k-th largest score, ordered tie
+//                          handling (smallest key index first), then the selected (score, index) pairs put in
+//                          order in shared memory, or their bits set.
 #pragma once
 #include "sm100_ptx.cuh"
 
@@ -59,123 +59,174 @@ struct TopkScoreParams {
   float* scores;       // [BH, n_blocks, s_stride]
   int* err;
   int n_blocks, kv_len, s_stride;
+  int k_tiles, q_tiles, n_tiles;       // 128-key tiles of a unit, 128-query-block tiles of a unit, score tiles in all
 };
 
 template <int D>
 struct TopkScoreCfg {
   static constexpr int kHalves = D / 64;
   static constexpr int kTileBytes = 128 * D * 2;
-  static constexpr int kStageBytes = 128 * 128 * 4;                   // fp32 score tile, reuses the operand tiles
-  static constexpr int kOffBar = (3 * kTileBytes > kStageBytes) ? 3 * kTileBytes : kStageBytes;
-  static constexpr int kSmemBytes = kOffBar + 64 + 1024;
-  static constexpr int kThreads = 160;                                // 4 epilogue warps + 1 load / issue warp
+  static constexpr int kStages = 4;
+  static constexpr int kOffK = 2 * kTileBytes;                        // behind the block means, hi and lo
+  static constexpr int kOffBar = kOffK + kStages * kTileBytes;
+  static constexpr int kSmemBytes = kOffBar + 256 + 1024;
+  static constexpr int kWarpProd = 8, kWarpIss = 9;
+  static constexpr int kThreads = 32 * 10;
 };
 
-// grid (key tiles, query-block tiles, BH).
+enum : int { TS_Q_FULL = 0, TS_Q_EMPTY = 1, TS_K_FULL = 2, TS_K_EMPTY = 6, TS_S_FULL = 10, TS_S_EMPTY = 12, TS_COUNT = 14 };
+
+// Score tiles (128 query blocks x 128 keys), key tiles of one query tile in a row, are cut into as many contiguous shares as
+// there are thread blocks (one per SM): the means are loaded once per share and unit, K streams through a ring, the
+// products go to two accumulators in turn, and a warpgroup each takes them from there to memory, a row per thread in
+// 32-byte pieces, which are whole sectors.  What is left is the writing of the scores.  12 heads, 256 query blocks x 32760
+// keys, D = 128 (402 MB): 0.113 ms; 0.146 with a thread block per tile and rows put together in shared memory.
+// Warps 0-3 / 4-7: even / odd tiles of the share, warp 8 TMA producer, warp 9 UMMA issuer.
 template <int D>
-__global__ void __launch_bounds__(TopkScoreCfg<D>::kThreads)
+__global__ void __launch_bounds__(TopkScoreCfg<D>::kThreads, 1)
 topk_scores_kernel(const __grid_constant__ CUtensorMap m_hi, const __grid_constant__ CUtensorMap m_lo,
                    const __grid_constant__ CUtensorMap mk, const TopkScoreParams p) {
   using Cfg = TopkScoreCfg<D>;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
   const uint32_t sbase = smem_u32(smem);
-  const uint32_t bar_full = sbase + Cfg::kOffBar, bar_done = bar_full + 8;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::kOffBar + 16);
-  AbortState* ab = reinterpret_cast<AbortState*>(smem + Cfg::kOffBar + 24);
+  auto bar = [&](int i) -> uint32_t { return sbase + Cfg::kOffBar + 8u * uint32_t(i); };
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(smem + Cfg::kOffBar + 8 * TS_COUNT);
+  AbortState* ab = reinterpret_cast<AbortState*>(smem + Cfg::kOffBar + 8 * TS_COUNT + 8);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int key0 = blockIdx.x * 128, qb0 = blockIdx.y * 128, bh = blockIdx.z;
+  const int from = int((long long)p.n_tiles * blockIdx.x / gridDim.x), to = int((long long)p.n_tiles * (blockIdx.x + 1) / gridDim.x);
 
   if (tid == 0) {
     ab->flag = 0;
-    mbar_init(bar_full, 1);
-    mbar_init(bar_done, 1);
+    mbar_init(bar(TS_Q_FULL), 1);
+    mbar_init(bar(TS_Q_EMPTY), 1);
+    for (int i = 0; i < Cfg::kStages; ++i) {
+      mbar_init(bar(TS_K_FULL + i), 1);
+      mbar_init(bar(TS_K_EMPTY + i), 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(bar(TS_S_FULL + i), 1);
+      mbar_init(bar(TS_S_EMPTY + i), 128);
+    }
     mbar_fence_init();
   }
-  if (warp == 4) {
+  if (warp == Cfg::kWarpProd) {
     __syncwarp();
-    tmem_alloc(smem_u32(tmem_slot), 128);
+    tmem_alloc(smem_u32(tmem_slot), 256);
     tmem_relinquish();
   }
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  const uint32_t a_hi = sbase, a_lo = sbase + Cfg::kTileBytes, b_k = sbase + 2 * Cfg::kTileBytes;
 
-  if (warp == 4) {
+  if (warp == Cfg::kWarpProd) {
     if (lane == 0) {
-      mbar_arrive_expect_tx(bar_full, 3 * Cfg::kTileBytes);
-      for (int h = 0; h < Cfg::kHalves; ++h) {
-        tma_load_3d(a_hi + h * 16384, &m_hi, bar_full, h * 64, qb0, bh);
-        tma_load_3d(a_lo + h * 16384, &m_lo, bar_full, h * 64, qb0, bh);
-        tma_load_3d(b_k + h * 16384, &mk, bar_full, h * 64, key0, bh);
+      tma_prefetch_desc(&m_hi);
+      tma_prefetch_desc(&m_lo);
+      tma_prefetch_desc(&mk);
+      bool ok = true;
+      int n_q = 0, g = 0;                                  // query tiles and K tiles requested so far
+      for (int i = from; i < to; ++i, ++g) {
+        const int row = i / p.k_tiles, unit = row / p.q_tiles;          // (unit, query tile)
+        if (i == from || i % p.k_tiles == 0) {
+          if (n_q > 0) ok = mbar_wait_relaxed(bar(TS_Q_EMPTY), (n_q - 1) & 1, ab, p.err, 3103);
+          if (!ok) break;
+          mbar_arrive_expect_tx(bar(TS_Q_FULL), 2 * Cfg::kTileBytes);
+          for (int h = 0; h < Cfg::kHalves; ++h) {
+            tma_load_3d(sbase + h * 16384, &m_hi, bar(TS_Q_FULL), h * 64, (row - unit * p.q_tiles) * 128, unit);
+            tma_load_3d(sbase + Cfg::kTileBytes + h * 16384, &m_lo, bar(TS_Q_FULL), h * 64, (row - unit * p.q_tiles) * 128, unit);
+          }
+          ++n_q;
+        }
+        const int st = g % Cfg::kStages, f = g / Cfg::kStages;
+        if (f > 0) ok = mbar_wait_relaxed(bar(TS_K_EMPTY + st), (f - 1) & 1, ab, p.err, 3104);
+        if (!ok) break;
+        mbar_arrive_expect_tx(bar(TS_K_FULL + st), Cfg::kTileBytes);
+        for (int h = 0; h < Cfg::kHalves; ++h)
+          tma_load_3d(sbase + Cfg::kOffK + st * Cfg::kTileBytes + h * 16384, &mk, bar(TS_K_FULL + st), h * 64,
+                      (i % p.k_tiles) * 128, unit);
+      }
+      if (!ok) {
+        // let the copies that are still in flight land before the thread block goes away
+        if (n_q > 0) mbar_wait_brief(bar(TS_Q_FULL), (n_q - 1) & 1);
+        for (int x = max(0, g - Cfg::kStages); x < g; ++x)
+          mbar_wait_brief(bar(TS_K_FULL + x % Cfg::kStages), (x / Cfg::kStages) & 1);
       }
     }
-    __syncwarp();
-    const bool ok = mbar_wait_warp(bar_full, 0, ab, p.err, 3101);
-    if (ok) {
+  } else if (warp == Cfg::kWarpIss) {
+    const uint32_t idesc = umma_idesc_bf16(128, 128, false);
+    bool ok = true;
+    int n_q = 0, g = 0;
+    for (int i = from; i < to && ok; ++i, ++g) {
+      if (i == from || i % p.k_tiles == 0) ok = mbar_wait_warp(bar(TS_Q_FULL), n_q++ & 1, ab, p.err, 3101);
+      const int st = g % Cfg::kStages, b = g & 1;
+      if (ok) ok = mbar_wait_warp(bar(TS_K_FULL + st), (g / Cfg::kStages) & 1, ab, p.err, 3105);
+      if (ok && g >= 2) ok = mbar_wait_warp(bar(TS_S_EMPTY + b), ((g >> 1) - 1) & 1, ab, p.err, 3106);
+      if (!ok) break;
       tc_fence_after();
-      const uint32_t idesc = umma_idesc_bf16(128, 128, false);
-      if (elect_one()) {               // one election for both products and the commit
+      const uint32_t kb = sbase + Cfg::kOffK + st * Cfg::kTileBytes;
+      if (elect_one()) {               // one election for both products and the commits
 #pragma unroll
         for (int part = 0; part < 2; ++part) {
-          const uint32_t a = part ? a_lo : a_hi;
 #pragma unroll
           for (int kk = 0; kk < D / 16; ++kk) {
             const uint32_t off = (kk / 4) * 16384 + (kk % 4) * 32;
-            umma_ss(tmem, umma_smem_desc_sw128(a + off, 16, 1024), umma_smem_desc_sw128(b_k + off, 16, 1024), idesc,
-                    (part | kk) ? 1u : 0u);
+            umma_ss(tmem + b * 128, umma_smem_desc_sw128(sbase + part * Cfg::kTileBytes + off, 16, 1024),
+                    umma_smem_desc_sw128(kb + off, 16, 1024), idesc, (part | kk) ? 1u : 0u);
           }
         }
-        umma_commit(bar_done);
+        umma_commit(bar(TS_S_FULL + b));
+        umma_commit(bar(TS_K_EMPTY + st));
+        if ((i + 1) % p.k_tiles == 0) umma_commit(bar(TS_Q_EMPTY));
       }
       __syncwarp();
     }
   } else {
-    // epilogue: one query-block row per thread -> shared-memory tile (16-byte chunks XOR-swizzled by
-    // row so that the row-per-thread stores and the row-per-warp loads are both conflict free)
-    const bool ok = mbar_wait(bar_done, 0, ab, p.err, 3102);
-    float* stage = reinterpret_cast<float*>(smem);
-    const int row = warp * 32 + lane;
-    if (ok) {
+    const int b = warp >> 2, wq = warp & 3;
+    const bool wide = (reinterpret_cast<uintptr_t>(p.scores) & 31) == 0;       // (rows are whole multiples of 512 bytes)
+    bool ok = true;
+    for (int i = from + b, f = 0; i < to; i += 2, ++f) {
+      ok = mbar_wait(bar(TS_S_FULL + b), f & 1, ab, p.err, 3102);
+      if (!ok) break;
       tc_fence_after();
+      const int row = i / p.k_tiles, unit = row / p.q_tiles, key0 = (i - row * p.k_tiles) * 128;
+      const int qb = (row - unit * p.q_tiles) * 128 + wq * 32 + lane;
+      float* dst = p.scores + (size_t(unit) * p.n_blocks + qb) * p.s_stride + key0;
+      const int live = p.kv_len - key0;                    // columns of this tile with a key
 #pragma unroll
       for (int cc = 0; cc < 4; ++cc) {
         uint32_t r[32];
-        tmem_ld32(tmem + (uint32_t(warp * 32) << 16) + cc * 32, r);
+        tmem_ld32(tmem + (uint32_t(wq * 32) << 16) + b * 128 + cc * 32, r);
         tmem_ld_wait();
-#pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const int chunk = cc * 8 + i;
-          float4 v = make_float4(__uint_as_float(r[4 * i]), __uint_as_float(r[4 * i + 1]), __uint_as_float(r[4 * i + 2]),
-                                 __uint_as_float(r[4 * i + 3]));
-          *reinterpret_cast<float4*>(stage + row * 128 + ((chunk ^ (row & 31)) << 2)) = v;
+        if (cc == 3) {
+          tc_fence_before();
+          mbar_arrive(bar(TS_S_EMPTY + b));
         }
-      }
-      tc_fence_before();
-    }
-    asm volatile("bar.sync 1, 128;" ::: "memory");        // the four epilogue warps
-    if (ok && !ab->flag) {
-      for (int r = warp; r < 128; r += 4) {
-        const int qb = qb0 + r;
-        if (qb >= p.n_blocks) break;
-        float4 v = *reinterpret_cast<const float4*>(stage + r * 128 + ((lane ^ (r & 31)) << 2));
-        const int key = key0 + lane * 4;
-        if (key >= p.s_stride) continue;
-        if (key + 0 >= p.kv_len) v.x = -INFINITY;
-        if (key + 1 >= p.kv_len) v.y = -INFINITY;
-        if (key + 2 >= p.kv_len) v.z = -INFINITY;
-        if (key + 3 >= p.kv_len) v.w = -INFINITY;
-        *reinterpret_cast<float4*>(p.scores + (size_t(bh) * p.n_blocks + qb) * p.s_stride + key) = v;
+        if (live < 128) {
+#pragma unroll
+          for (int e = 0; e < 32; ++e)
+            if (cc * 32 + e >= live) r[e] = __float_as_uint(-INFINITY);
+        }
+        if (qb < p.n_blocks) {
+#pragma unroll
+          for (int e = 0; e < 32; e += 8) {
+            if (wide) {
+              st_global_v8(dst + cc * 32 + e, &r[e]);
+            } else {
+              *reinterpret_cast<uint4*>(dst + cc * 32 + e) = make_uint4(r[e], r[e + 1], r[e + 2], r[e + 3]);
+              *reinterpret_cast<uint4*>(dst + cc * 32 + e + 4) = make_uint4(r[e + 4], r[e + 5], r[e + 6], r[e + 7]);
+            }
+          }
+        }
       }
     }
   }
   tc_fence_before();
   __syncthreads();
-  if (warp == 4) {
+  if (warp == Cfg::kWarpProd) {
     __syncwarp();
-    tmem_dealloc(tmem, 128);
+    tmem_dealloc(tmem, 256);
   }
 }
 
@@ -193,22 +244,32 @@ constexpr int kSelThreads = 512;
 constexpr int kSelBins = 2048;
 constexpr uint32_t kSelBinSort = 64;         // entries of one bin that are ordered by counting
 
-// grid (rows), kSelThreads threads, dynamic shared memory = 10 * pow2ceil(k) bytes.  Row r of `scores`
-// has n entries (stride s_stride, a multiple of 4, rows 16-byte aligned); writes the indices of its k
-// largest entries in descending score order (equal scores: smaller index first) to idx[r][0..k) and k
-// to cnt[r].  Requires 1 <= k <= n.  Every sweep reads the row from global memory (L2 after the first;
-// keeping the row in shared memory instead allows one CTA per SM only and measured slower).
+// Entries that the selection collects at most.  A quarter more than k leaves room for a threshold that is read off a sample
+// (and 1024 for the small k, whose share of the sample is a few entries); a power of two at least k is what the sort needs.
+inline int select_capacity(int k) {
+  int pow2 = 2;
+  while (pow2 < k) pow2 <<= 1;
+  const int wide = (k + (k >> 2) + 63) & ~63;
+  return wide > pow2 ? (wide > 1024 ? wide : 1024) : (pow2 > 1024 ? pow2 : 1024);
+}
+
+// grid (rows), kSelThreads threads.  Row r of `scores` has n entries (stride s_stride, a multiple of 4, rows 16-byte
+// aligned).  The k largest (equal scores: smaller index first), 1 <= k <= n:
+// BITS = false: their indices in descending score order to idx[r][0..k), k to cnt[r], list_stride to the slots behind.
+//   Dynamic shared memory: 8 * (cap + kSelBinSort) + 2 * cap bytes.
+// BITS = true: their bits set in row r of `bits` (row_words words), the others clear; what an attention step needs of a
+//   selection, without the order.  Dynamic shared memory: 8 * (cap + kSelBinSort) + 4 * row_words bytes.
 //
-// Selection works on the order-preserving unsigned image of the scores.  A first sweep finds the
-// smallest and largest key of the row; each following sweep histograms the keys of the current
-// interval into 2048 equal bins (a plain byte-wise radix would put almost every score of a row into
-// two or three bins of its leading byte and serialise the shared-memory counters), picks the bin
-// that holds the k-th largest and narrows the interval to it, until the bin and everything above it
-// fit the sort buffer (usually after one histogram sweep) or the bins are one key wide.
-__global__ void __launch_bounds__(kSelThreads)
-topk_select_kernel(const float* __restrict__ scores, int s_stride, int n, int k, int k_pow2, int* __restrict__ idx,
-                   int* __restrict__ cnt, int list_stride) {
-  extern __shared__ unsigned long long sel[];            // (key << 32 | ~index), k_pow2 entries; then k_pow2 slots
+// A sample of the row, 16 of every 128 bytes, gives a score that more than k and fewer than cap entries reach -- nearly
+// always; one sweep then collects those, and the count says whether it was so.  Rows where it was not go the general way
+// (below), which needs the range of the keys, one to three histogram sweeps and a sweep that collects.  3072 rows of
+// 32760 scores, k = 3276: 0.449 -> 0.235 ms with bits (the general way and the counting of places, all rows).
+template <bool BITS>
+__global__ void __launch_bounds__(kSelThreads, 3)
+topk_select_kernel(const float* __restrict__ scores, int s_stride, int n, int k, int k_pow2, int cap, int* __restrict__ idx,
+                   int* __restrict__ cnt, int list_stride, uint32_t* __restrict__ bits, int row_words) {
+  // (key << 32 | ~index), cap entries and room for a bin's; then cap slots, or the row's bits
+  extern __shared__ unsigned long long sel[];
   __shared__ int hist[kSelBins];
   __shared__ uint32_t s_lo, s_hi, s_max;
   __shared__ int s_rem, s_ties, s_count, s_base;
@@ -218,6 +279,9 @@ topk_select_kernel(const float* __restrict__ scores, int s_stride, int n, int k,
   const float* row = scores + size_t(blockIdx.x) * s_stride;
   const float4* row4 = reinterpret_cast<const float4*>(row);
   const int n4 = (n + 3) >> 2;
+  unsigned long long* const after = sel + cap + kSelBinSort;
+  uint16_t* slot = reinterpret_cast<uint16_t*>(after);
+  uint32_t* row_bits = reinterpret_cast<uint32_t*>(after);
 
   // One sweep over the row, four 16-byte loads in flight per thread; f(key, index, live) per entry.
   // The trip count is the same for every thread, so f may use full-warp collectives.
@@ -238,6 +302,228 @@ topk_select_kernel(const float* __restrict__ scores, int s_stride, int n, int k,
       }
     }
   };
+  // smallest and largest key over the block -> s_lo, s_hi
+  auto key_range = [&](uint32_t kmin, uint32_t kmax) {
+    kmin = __reduce_min_sync(0xffffffffu, kmin);
+    kmax = __reduce_max_sync(0xffffffffu, kmax);
+    if (lane == 0) { red_lo[warp] = kmin; red_hi[warp] = kmax; }
+    __syncthreads();
+    if (tid == 0) {
+      uint32_t a = red_lo[0], b = red_hi[0];
+      for (int w = 1; w < kSelThreads / 32; ++w) { a = min(a, red_lo[w]); b = max(b, red_hi[w]); }
+      s_lo = a;
+      s_hi = b;
+    }
+    __syncthreads();
+  };
+  auto clear_hist = [&]() {
+    for (int i = tid; i < kSelBins; i += kSelThreads) hist[i] = 0;
+  };
+  // Exclusive sums over the bins into hist, four bins per thread; returns the fullest bin's count.
+  auto scan_hist = [&]() -> uint32_t {
+    static_assert(kSelBins == 4 * kSelThreads, "four bins per thread");
+    int c[4], sum = 0, most = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      c[u] = hist[4 * tid + u];
+      sum += c[u];
+      most = max(most, c[u]);
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int t = __shfl_up_sync(0xffffffffu, incl, o);
+      if (lane >= o) incl += t;
+    }
+    most = __reduce_max_sync(0xffffffffu, most);
+    if (lane == 31) warp_tot[warp] = incl;
+    if (lane == 0) red_hi[warp] = uint32_t(most);
+    __syncthreads();
+    int start = incl - sum;
+    uint32_t fullest = 0;
+#pragma unroll
+    for (int w = 0; w < kSelThreads / 32; ++w) {
+      if (w < warp) start += warp_tot[w];
+      fullest = max(fullest, red_hi[w]);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      hist[4 * tid + u] = start;
+      start += c[u];
+    }
+    __syncthreads();
+    return fullest;
+  };
+  // bins of equal score width from f_hi down to f_lo; false where the scores do not spread over a finite range (f_hi == f_lo
+  // gives an infinite factor, so does a range under about 1e-35, an infinite score a zero or NaN)
+  float f_hi = 0.f, to_bin = 0.f;
+  auto set_bins = [&](uint32_t key_hi, uint32_t key_lo) -> bool {
+    f_hi = float_of_order_key(key_hi);
+    to_bin = float(kSelBins - 1) / (f_hi - float_of_order_key(key_lo));
+    return to_bin > 0.f && to_bin < 1e30f;
+  };
+  auto bin_of_key = [&](uint32_t key) -> int { return max(0, min(kSelBins - 1, int((f_hi - float_of_order_key(key)) * to_bin))); };
+
+  // The k largest of the m >= k entries in sel, whose keys lie in [key_lo, key_hi], by counting: the entries are counted into
+  // 2048 bins of equal width over their range of scores (a monotone map, so a larger bin holds smaller scores), every
+  // entry gets a slot in its bin, and inside a bin -- a few entries -- an entry's place is the number of larger ones.
+  // Five barriers where a bitonic sort of 4096 entries takes 78 passes: 3276 of 32760 keys for 3072 rows, the whole
+  // selection 1.017 -> 0.569 ms (8192 keys 1.864 -> 1.001 ms).  False, and nothing written, for scores that pile up in a
+  // few bins (equal or infinite ones, or one far above all others), where counting inside the bins would be quadratic:
+  // with kSelBinSort = 256 one score at 30 deviations takes 3.2 ms at 8192 keys, by the sort 1.55.
+  auto finish_by_counting = [&](int m, uint32_t key_hi, uint32_t key_lo) -> bool {
+    if (!set_bins(key_hi, key_lo)) return false;
+    clear_hist();
+    if (tid == 0) s_count = 0;
+    __syncthreads();
+    for (int i = tid; i < m; i += kSelThreads) atomicAdd(&hist[bin_of_key(uint32_t(sel[i] >> 32))], 1);
+    __syncthreads();
+    if (scan_hist() > kSelBinSort) return false;
+    // hist[b] is the start of bin b
+    if constexpr (BITS) {
+      for (int i = tid; i < row_words; i += kSelThreads) row_bits[i] = 0u;
+      __syncthreads();
+      auto set_bit = [&](unsigned long long e) {
+        const uint32_t i = ~uint32_t(e & 0xffffffffull);
+        atomicOr(&row_bits[i >> 5], 1u << (i & 31));
+      };
+      // bins that end at k or before are taken whole, the entries of the one that k falls into are compared
+      unsigned long long* edge = sel + cap;
+      for (int i = tid; i < m; i += kSelThreads) {
+        const unsigned long long e = sel[i];
+        const int b = bin_of_key(uint32_t(e >> 32));
+        if ((b + 1 < kSelBins ? hist[b + 1] : m) <= k) set_bit(e);
+        else if (hist[b] < k) edge[atomicAdd(&s_count, 1)] = e;
+      }
+      __syncthreads();
+      const int c = s_count;
+      if (tid < c) {
+        const unsigned long long e = edge[tid];
+        int place = hist[bin_of_key(uint32_t(e >> 32))];
+        for (int j = 0; j < c; ++j) place += edge[j] > e ? 1 : 0;
+        if (place < k) set_bit(e);
+      }
+      __syncthreads();
+      uint32_t* dst = bits + size_t(blockIdx.x) * row_words;
+      for (int i = tid; i < row_words; i += kSelThreads) dst[i] = row_bits[i];
+    } else {
+      for (int i = tid; i < m; i += kSelThreads) slot[atomicAdd(&hist[bin_of_key(uint32_t(sel[i] >> 32))], 1)] = uint16_t(i);
+      __syncthreads();
+      // hist[b] is now the end of bin b, which is where bin b + 1 starts
+      int* dst = idx + size_t(blockIdx.x) * list_stride;
+      for (int i = tid; i < m; i += kSelThreads) {
+        const unsigned long long e = sel[i];
+        const int b = bin_of_key(uint32_t(e >> 32)), s0 = b ? hist[b - 1] : 0, s1 = hist[b];
+        int place = s0;
+        for (int j = s0; j < s1; ++j) place += sel[slot[j]] > e ? 1 : 0;
+        if (place < k) dst[place] = int(~uint32_t(e & 0xffffffffull));
+      }
+      for (int i = k + tid; i < list_stride; i += kSelThreads) dst[i] = list_stride;
+      if (tid == 0) cnt[blockIdx.x] = k;
+    }
+    return true;
+  };
+
+  // ---- the short way
+  {
+    const int m4 = (n4 + 7) >> 3;                          // float4s of the sample
+    uint32_t kmin = 0xffffffffu, kmax = 0u;
+    auto sample = [&](auto&& f) {
+      for (int i = tid; i < m4; i += kSelThreads) {
+        const float4 v = row4[8 * i];
+        const float x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (32 * i + e < n) f(float_order_key(x[e]));
+      }
+    };
+    sample([&](uint32_t key) {
+      kmin = min(kmin, key);
+      kmax = max(kmax, key);
+    });
+    key_range(kmin, kmax);
+    const uint32_t lo_key = s_lo, hi_key = s_hi;
+    const int m = 4 * (m4 - 1) + min(4, n - 32 * (m4 - 1));
+    // the sample's rank of a score that (k + cap) / 2 entries of the row reach
+    const int rank = int((long long)(k + cap) * m / (2 * n));
+    if (rank >= 1 && rank < m && set_bins(hi_key, lo_key)) {
+      clear_hist();
+      if (tid == 0) { s_count = 0; s_max = 0u; s_rem = kSelBins; }
+      __syncthreads();
+      sample([&](uint32_t key) { atomicAdd(&hist[bin_of_key(key)], 1); });
+      __syncthreads();
+      scan_hist();
+      // the first bin that starts at or past that rank: its upper edge is the threshold
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int b = 4 * tid + u;
+        if (b > 0 && hist[b] >= rank && hist[b - 1] < rank) s_rem = b;
+      }
+      __syncthreads();
+      if (s_rem < kSelBins) {
+        const uint32_t from = float_order_key(f_hi - float(s_rem) / to_bin);
+        uint32_t top = 0u;
+        for (int base = 0; base < n4; base += 4 * kSelThreads) {
+          float4 v[4];
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int j = base + u * kSelThreads + tid;
+            v[u] = (j < n4) ? row4[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+          }
+          uint32_t take = 0u;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const int j = base + u * kSelThreads + tid;
+            const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e)
+              if (float_order_key(x[e]) >= from && 4 * j + e < n) take |= 1u << (4 * u + e);
+          }
+          const int c = __popc(take);
+          int incl = c;
+#pragma unroll
+          for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
+          }
+          int at = 0;
+          if (lane == 31 && incl > 0) at = atomicAdd(&s_count, incl);
+          at = __shfl_sync(0xffffffffu, at, 31) + incl - c;
+#pragma unroll
+          for (int u = 0; u < 4; ++u) {
+            const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              if ((take >> (4 * u + e)) & 1u) {
+                const uint32_t key = float_order_key(x[e]);
+                top = max(top, key);
+                if (at < cap)
+                  sel[at] = (static_cast<unsigned long long>(key) << 32) |
+                            uint32_t(~uint32_t(4 * (base + u * kSelThreads + tid) + e));
+                ++at;
+              }
+            }
+          }
+        }
+        top = __reduce_max_sync(0xffffffffu, top);
+        if (lane == 0) atomicMax(&s_max, top);
+        __syncthreads();
+        const int got = s_count;
+        const uint32_t max_key = s_max;
+        __syncthreads();
+        if (got >= k && got <= cap && finish_by_counting(got, max_key, from)) return;
+      }
+    }
+    __syncthreads();
+  }
+
+  // ---- The general way.  Every sweep reads the row from global memory (L2 after the first; keeping the row in shared
+  // memory instead allows one thread block per SM only and measured slower).  Selection works on the order-preserving
+  // unsigned image of the scores.  A first sweep finds the smallest and largest key of the row; each following sweep
+  // histograms the keys of the current interval into 2048 equal bins (a plain byte-wise radix would put almost every score
+  // of a row into two or three bins of its leading byte and serialise the shared-memory counters), picks the bin that
+  // holds the k-th largest and narrows the interval to it, until the bin and everything above it fit the sort buffer
+  // (usually after one histogram sweep) or the bins are one key wide.
   // ---- key range of the row
   uint32_t kmin = 0xffffffffu, kmax = 0u;
   sweep([&](uint32_t key, int, bool live) {
@@ -246,16 +532,9 @@ topk_select_kernel(const float* __restrict__ scores, int s_stride, int n, int k,
       kmax = max(kmax, key);
     }
   });
-  kmin = __reduce_min_sync(0xffffffffu, kmin);
-  kmax = __reduce_max_sync(0xffffffffu, kmax);
-  if (lane == 0) { red_lo[warp] = kmin; red_hi[warp] = kmax; }
-  __syncthreads();
+  key_range(kmin, kmax);
   if (tid == 0) {
-    uint32_t a = red_lo[0], b = red_hi[0];
-    for (int w = 1; w < kSelThreads / 32; ++w) { a = min(a, red_lo[w]); b = max(b, red_hi[w]); }
-    s_lo = a;
-    s_hi = b;
-    s_max = b;
+    s_max = s_hi;
     s_rem = k;
   }
   __syncthreads();
@@ -352,75 +631,10 @@ topk_select_kernel(const float* __restrict__ scores, int s_stride, int n, int k,
   }
   __syncthreads();
 
-  // ---- descending order.  The m collected entries are counted into 2048 bins of equal width over their range of
-  // scores (a monotone map, so a larger bin holds smaller scores), every entry gets a slot in its bin, and inside a
-  // bin -- a few entries -- an entry's place is the number of larger ones.  Five barriers where a bitonic sort of
-  // 4096 entries takes 78 passes: 3276 of 32760 keys for 3072 rows, the whole selection 1.017 -> 0.569 ms (8192 keys
-  // 1.864 -> 1.001 ms, although the slots leave room for two rows on an SM instead of three).  The sort stays for scores
-  // that pile up in a few bins (equal or infinite ones, or one far above all others), where counting inside the bins
-  // would be quadratic: with kSelBinSort = 256 one score at 30 deviations takes 3.2 ms at 8192 keys, by the sort 1.55.
   const int m = (n_gt + s_ties <= k_pow2) ? n_gt + s_ties : k;
-  const float f_hi = float_of_order_key(s_max), f_lo = float_of_order_key(kth);
-  const float to_bin = float(kSelBins - 1) / (f_hi - f_lo);
-  auto bin_of = [&](unsigned long long e) -> int {
-    return min(kSelBins - 1, int((f_hi - float_of_order_key(uint32_t(e >> 32))) * to_bin));
-  };
-  // (f_hi == f_lo gives an infinite factor; so does a range under about 1e-35; an infinite score a zero or NaN)
-  const bool spread = to_bin > 0.f && to_bin < 1e30f;
-  uint16_t* slot = reinterpret_cast<uint16_t*>(sel + k_pow2);
-  if (spread) {
-    for (int i = tid; i < kSelBins; i += kSelThreads) hist[i] = 0;
-    __syncthreads();
-    for (int i = tid; i < m; i += kSelThreads) atomicAdd(&hist[bin_of(sel[i])], 1);
-    __syncthreads();
-    static_assert(kSelBins == 4 * kSelThreads, "four bins per thread");
-    int c[4], sum = 0, most = 0;
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      c[u] = hist[4 * tid + u];
-      sum += c[u];
-      most = max(most, c[u]);
-    }
-    int incl = sum;
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const int t = __shfl_up_sync(0xffffffffu, incl, o);
-      if (lane >= o) incl += t;
-    }
-    most = __reduce_max_sync(0xffffffffu, most);
-    if (lane == 31) warp_tot[warp] = incl;
-    if (lane == 0) red_hi[warp] = uint32_t(most);
-    __syncthreads();
-    int start = incl - sum;
-    uint32_t fullest = 0;
-#pragma unroll
-    for (int w = 0; w < kSelThreads / 32; ++w) {
-      if (w < warp) start += warp_tot[w];
-      fullest = max(fullest, red_hi[w]);
-    }
-    if (fullest <= kSelBinSort) {
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        hist[4 * tid + u] = start;
-        start += c[u];
-      }
-      __syncthreads();
-      for (int i = tid; i < m; i += kSelThreads) slot[atomicAdd(&hist[bin_of(sel[i])], 1)] = uint16_t(i);
-      __syncthreads();
-      // hist[b] is now the end of bin b, which is where bin b + 1 starts
-      int* dst = idx + size_t(blockIdx.x) * list_stride;
-      for (int i = tid; i < m; i += kSelThreads) {
-        const unsigned long long e = sel[i];
-        const int b = bin_of(e), s0 = b ? hist[b - 1] : 0, s1 = hist[b];
-        int place = s0;
-        for (int j = s0; j < s1; ++j) place += sel[slot[j]] > e ? 1 : 0;
-        if (place < k) dst[place] = int(~uint32_t(e & 0xffffffffull));
-      }
-      for (int i = k + tid; i < list_stride; i += kSelThreads) dst[i] = list_stride;
-      if (tid == 0) cnt[blockIdx.x] = k;
-      return;
-    }
-  }
+  const uint32_t key_top = s_max;
+  if (finish_by_counting(m, key_top, kth)) return;
+  __syncthreads();
 
   // ---- bitonic sort, descending: the first k entries are the answer.  The passes of strides up to 32 stay inside groups
   // of 64 entries: a warp takes a group through all of them in registers, two entries a lane, and only the passes
@@ -471,10 +685,22 @@ topk_select_kernel(const float* __restrict__ scores, int s_stride, int n, int k,
     }
     in_group(size, size);
   }
-  int* dst = idx + size_t(blockIdx.x) * list_stride;
-  for (int i = tid; i < k; i += kSelThreads) dst[i] = int(~uint32_t(sel[i] & 0xffffffffull));
-  for (int i = k + tid; i < list_stride; i += kSelThreads) dst[i] = list_stride;
-  if (tid == 0) cnt[blockIdx.x] = k;
+  if constexpr (BITS) {
+    for (int i = tid; i < row_words; i += kSelThreads) row_bits[i] = 0u;
+    __syncthreads();
+    for (int i = tid; i < k; i += kSelThreads) {
+      const uint32_t key = ~uint32_t(sel[i] & 0xffffffffull);
+      atomicOr(&row_bits[key >> 5], 1u << (key & 31));
+    }
+    __syncthreads();
+    uint32_t* dst = bits + size_t(blockIdx.x) * row_words;
+    for (int i = tid; i < row_words; i += kSelThreads) dst[i] = row_bits[i];
+  } else {
+    int* dst = idx + size_t(blockIdx.x) * list_stride;
+    for (int i = tid; i < k; i += kSelThreads) dst[i] = int(~uint32_t(sel[i] & 0xffffffffull));
+    for (int i = k + tid; i < list_stride; i += kSelThreads) dst[i] = list_stride;
+    if (tid == 0) cnt[blockIdx.x] = k;
+  }
 }
 
 }  // namespace fg

@@ -41,6 +41,10 @@ class nvtx_range:
 # mask caches (python/spattn/mask_utils.py:17-98): decide on which diffusion runs the mask is
 # rebuilt and hand the cached lists to the sparse steps in between
 # ------------------------------------------------------------------------------------------------
+def _is_method(bound, obj, func) -> bool:
+    return getattr(bound, "__self__", None) is obj and getattr(bound, "__func__", None) is func
+
+
 class NaiveMaskCache:
     """Keeps whatever the build step produced, per layer, on the device."""
 
@@ -94,14 +98,19 @@ class CompressedBitMaskCache(BitMaskCache):
         """What an attention step reads its lists with: get_lists, unless a program has put a get_mask_from_cache of
         its own in a subclass, in this class or on the object."""
         read = self.get_mask_from_cache
-        own = getattr(read, "__self__", None) is self and \
-            getattr(read, "__func__", None) is CompressedBitMaskCache._own_reading
-        return self.get_lists if own else read
+        return self.get_lists if _is_method(read, self, CompressedBitMaskCache._own_reading) else read
 
     def get_lists(self, layer):
         """The same lists for the attention operator alone: slots past the counts hold anything."""
         packed, seq_len = self.cache[layer]
         return _packedmask_to_lists(packed, seq_len)
+
+    _own_list_reader, _own_lists = list_reader, get_lists
+
+    def reads_bits(self):
+        """An attention step may go by the kept bits themselves: nothing of what hands out the lists has been replaced."""
+        return _is_method(self.list_reader, self, CompressedBitMaskCache._own_list_reader) and \
+            _is_method(self.list_reader(), self, CompressedBitMaskCache._own_lists)
 
     def update_cache(self, layer, mask, seq_len):
         self.cache[layer] = (pack(mask), seq_len)
@@ -327,13 +336,6 @@ def qk_indexmask_cuda(q, k, thresh, blocksz=128):
         return packedmask_to_indexmask_cuda(packed, k.shape[2])
 
 
-def _qk_token_lists(q, k, thresh):
-    """qk_indexmask_cuda(q, k, thresh) for the attention operator alone: slots past the counts hold anything."""
-    packed = _qk_packed_token_mask(q, k, thresh)
-    with nvtx_range("fgattn.mask_to_lists"):
-        return _packedmask_to_lists(packed, k.shape[2])
-
-
 # ------------------------------------------------------------------------------------------------
 # alternative selectors (python/spattn/mask_utils.py:385-417)
 # ------------------------------------------------------------------------------------------------
@@ -356,3 +358,16 @@ def qk_topkmask_indices(q, k, select_k, B=None, H=None, S=None, D=None, BLOCKSZ=
     spattn_interface.topk_indices(kv_indices, kv_num_indices, q.contiguous(), k.contiguous(), int(select_k),
                                   int(BLOCKSZ))
     return kv_indices, kv_num_indices
+
+
+# keys per row of a selection handed over as bits, which are put together in shared memory beside the selected entries
+MAX_PACKED_SELECTION = 524288
+
+
+def _qk_topk_packed(q, k, select_k, blocksz=128):
+    """The keys of qk_topkmask_indices as one bit per key (uint8, pad128(S_kv) / 8 bytes a row): for an attention step,
+    which does not ask in what order they were selected."""
+    B, H, S, _ = q.shape
+    packed = torch.empty((B, H, (S + blocksz - 1) // blocksz, _pad128(k.shape[2]) // 8), dtype=torch.uint8, device=q.device)
+    spattn_interface.topk_packed(packed, q.contiguous(), k.contiguous(), int(select_k), int(blocksz))
+    return packed

@@ -61,13 +61,23 @@ def _sparse(out, query, key, value, mask, blocksz=128):
     return out
 
 
+def _sparse_bits(out, query, key, value, packed, n_valid):
+    """One sparse step on a token mask of one bit per key, of which the first n_valid (None: all) count."""
+    if key.shape[2] >= 1 << 21:                            # more than the packed form counts
+        return _sparse(out, query, key, value, mask_utils._packedmask_to_lists(packed, n_valid))
+    with mask_utils.nvtx_range("fgattn.sparse_attention"):
+        spattn_interface.sp_attn_packed(out, query.contiguous(), key.contiguous(), value.contiguous(), packed.contiguous(),
+                                        packed.shape[-1] * 8 if n_valid is None else n_valid)
+    return out
+
+
 def attn_computed_with_sparse_mask_cuda(query, key, value, *args, **kwargs):
     """Build the mask from (query, key) and run the sparse kernel with it
     (sparseattn_functionals.py:61-69)."""
     if kwargs["blocksz"] == 128:
-        mask = mask_utils._qk_token_lists(query, key, kwargs["thresh"])
-    else:
-        mask = mask_utils.qk_indexmask_cuda(query, key, kwargs["thresh"], blocksz=kwargs["blocksz"])
+        packed = mask_utils._qk_packed_token_mask(query, key, kwargs["thresh"])
+        return _sparse_bits(_out(query), query, key, value, packed, key.shape[2])
+    mask = mask_utils.qk_indexmask_cuda(query, key, kwargs["thresh"], blocksz=kwargs["blocksz"])
     return _sparse(_out(query), query, key, value, mask)
 
 
@@ -75,6 +85,9 @@ def attn_topkmask_cuda(query, key, value, current_layer=None, ditrun=None, *args
     """Top-k key selection per 128-row query block, then the token-list sparse kernel
     (sparseattn_functionals.py:39-48)."""
     select_k = kwargs.get("select_k") or query.shape[2]
+    if key.shape[2] <= mask_utils.MAX_PACKED_SELECTION:
+        packed = mask_utils._qk_topk_packed(query, key, select_k, kwargs.get("blocksz", 128))
+        return _sparse_bits(_out(query), query, key, value, packed, key.shape[2])
     mask = mask_utils.qk_topkmask_indices(query, key, select_k, blocksz=kwargs.get("blocksz", 128))
     return _sparse(_out(query), query, key, value, mask)
 
@@ -129,6 +142,8 @@ def bitmaskcached_attn_cuda(query, key, value, current_layer, ditrun, *args, **k
         mask_cache.update_cache(current_layer, mask, key.shape[2])
         return out
     compressed = isinstance(mask_cache, mask_utils.CompressedBitMaskCache)
+    if compressed and mask_cache.reads_bits():
+        return _sparse_bits(_out(query), query, key, value, *mask_cache.cache[current_layer])
     read = mask_cache.list_reader() if compressed else mask_cache.get_mask_from_cache
     return _sparse(_out(query), query, key, value, read(current_layer)[:2])
 

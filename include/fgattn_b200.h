@@ -142,6 +142,16 @@ int fgattn_sp_attn(void* o, const void* q, const void* k, const void* v, const i
                    const int* kv_num_indices, int mask_stride, int batch, int heads, int seq, int D, int kv_rows,
                    float scale, void* workspace, size_t workspace_bytes, void* stream);
 
+/* The same attention on a packed mask (one bit per key, see fgattn_pack_mask): query block i of a unit attends to the keys
+ * whose bits are set in its row of row_bytes bytes, packed [B,H,ceil(seq/128),row_bytes]; bits from min(n_valid, kv_rows)
+ * on do not count.  Keys that two neighbouring query blocks both keep are gathered once for the two.  `workspace`
+ * (scratch) of fgattn_sp_attn_packed_workspace_bytes is needed.  kv_rows < 2^21.  Same result within rounding as fgattn_sp_attn on the
+ * lists of fgattn_packedmask_to_lists. */
+size_t fgattn_sp_attn_packed_workspace_bytes(int batch, int heads, int seq, int kv_rows);
+int fgattn_sp_attn_packed(void* o, const void* q, const void* k, const void* v, const unsigned char* packed, int row_bytes,
+                          int n_valid, int batch, int heads, int seq, int D, int kv_rows, float scale, void* workspace,
+                          size_t workspace_bytes, void* stream);
+
 /* ---- 64x64 block granularity --------------------------------------------------------------- */
 
 /* Bytes of scratch that fgattn_block_index_lists wants in order to process all batch*heads units
@@ -294,6 +304,12 @@ size_t fgattn_topk_scratch_bytes(int batch, int heads, int seq, int D, int block
 int fgattn_topk_indices(int* kv_indices, int* kv_num_indices, int list_stride, const void* q, const void* k,
                         int select_k, int batch, int heads, int seq, int D, int blocksz, int kv_rows, int kv_seq_len,
                         float scale, void* scratch, size_t scratch_bytes, void* stream);
+
+/* The same selection as a packed mask (one bit per key, rows of row_bytes bytes, a multiple of 4 and at least
+ * kv_seq_len / 8): what fgattn_sp_attn_packed takes.  packed [B,H,ceil(seq/blocksz),row_bytes], 4-byte aligned. */
+int fgattn_topk_packed(unsigned char* packed, int row_bytes, const void* q, const void* k, int select_k, int batch, int heads,
+                       int seq, int D, int blocksz, int kv_rows, int kv_seq_len, float scale, void* scratch,
+                       size_t scratch_bytes, void* stream);
 
 /* ---- self-test ------------------------------------------------------------------------------- */
 

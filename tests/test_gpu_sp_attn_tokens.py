@@ -245,3 +245,66 @@ def test_output_rows_at_the_edges(S, D):
     capi.check()
     _close(o, orc.sp_attn_tokens(q, k, v, idx, cnt, 128))
     assert torch.all(buf[n:] == 7.0)
+
+
+@pytest.mark.parametrize("S,D,n_kv,n_valid,row_bytes", [(256, 128, 1500, 1500, 192), (640, 64, 1500, 1400, 188), (1000, 128, 1500, 9999, 189),
+                                                       (128, 64, 33, 33, 5), (300, 128, 9000, 9000, 1125)])
+def test_packed_mask_and_shared_tiles(S, D, n_kv, n_valid, row_bytes):
+    """sp_attn_packed: keys that both blocks of a pair keep are gathered once, in whole tiles of 128 (packed_pairs_kernel).
+    Masks with every kind of overlap, rows of whole and of broken words, bits past the last key and past n_valid, against
+    the oracle and against sp_attn on the lists of the same bits."""
+    import numpy as np
+    import fgattn_tk_cuda_b200.spattn  # noqa: F401  (registers torch.ops.cuda_attn)
+    from oracle import fgattn_oracle as orc
+    capi = _capi()
+    # keys of the first block, of the second, of both
+    kinds = [(700, 700, 700), (127, 127, 127), (128, 128, 128), (255, 129, 129), (700, 300, 0), (900, 900, 128), (0, 500, 0),
+             (513, 640, 400), (n_kv, n_kv, n_kv), (256, 900, 256), (500, 0, 0), (0, 0, 0), (129, 1, 1)]
+    nb = (S + 127) // 128
+    pairs = (nb + 1) // 2
+    B, H = 1, -(-len(kinds) // pairs)
+    g = torch.Generator().manual_seed(S + n_kv)
+    q = torch.randn(B, H, S, D, generator=g).to(torch.bfloat16)
+    k, v = (torch.randn(B, H, n_kv, D, generator=g).to(torch.bfloat16) for _ in range(2))
+    bits = torch.zeros(H * 2 * pairs, 8 * row_bytes, dtype=torch.bool)
+    for i in range(H * pairs):
+        n0, n1, both = (min(n, n_kv) for n in kinds[i % len(kinds)])
+        perm = torch.randperm(n_kv, generator=g)
+        bits[2 * i, perm[:n0]] = True
+        bits[2 * i + 1, torch.cat([perm[:both], perm[n0:n0 + n1 - both]])] = True
+    bits[:, n_kv:] = True
+    bits = bits.view(H, 2 * pairs, -1)[:, :nb].contiguous()
+    packed = torch.from_numpy(np.packbits(bits.numpy(), axis=-1, bitorder="little")).view(B, H, nb, row_bytes)
+    limit = min(n_valid, n_kv)
+    stride = 128 * ((n_kv + 127) // 128)
+    idx, cnt = _lists_from_mask(bits[None, ..., :limit], stride)
+    o, again, lists = (torch.full((B, H, S, D), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(3))
+    args = (q.cuda(), k.cuda(), v.cuda())
+    torch.ops.cuda_attn.sp_attn_packed(o, *args, packed.cuda(), n_valid)
+    torch.ops.cuda_attn.sp_attn_packed(again, *args, packed.cuda(), n_valid)
+    torch.ops.cuda_attn.sp_attn(lists, *args, idx.cuda(), cnt.cuda())
+    capi.check()
+    _close(o, orc.sp_attn_tokens(q, k, v, idx, cnt, 128))
+    # the keys' order differs, so does the rounding of the probabilities and of the output: 2^-8 of values up to about 1
+    _close(o, lists, 8e-3, 5e-4)
+    assert torch.equal(o, again)
+
+
+def test_packed_mask_of_more_than_a_sweep():
+    """Rows of more than 32768 bits (packed_pairs_kernel takes 1024 words a sweep): against sp_attn on the lists."""
+    import fgattn_tk_cuda_b200.spattn  # noqa: F401  (registers torch.ops.cuda_attn)
+    from fgattn_tk_cuda_b200.spattn import mask_utils as mu
+    B, H, S, D, n_kv = 1, 3, 300, 64, 70001
+    g = torch.Generator(device="cuda").manual_seed(3)
+    q = torch.randn(B, H, S, D, generator=g, device="cuda").to(torch.bfloat16)
+    k, v = (torch.randn(B, H, n_kv, D, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    common = torch.rand(B, H, 1, 70016, generator=g, device="cuda") < 0.02
+    bits = common | (torch.rand(B, H, 3, 70016, generator=g, device="cuda") < 0.005)
+    bits[..., 30000:31000] = True
+    packed = mu.pack(bits)
+    o, lists = torch.full_like(q, float("nan")), torch.full_like(q, float("nan"))
+    torch.ops.cuda_attn.sp_attn_packed(o, q, k, v, packed, n_kv)
+    idx, cnt = mu.packedmask_to_indexmask_cuda(packed, n_kv)
+    torch.ops.cuda_attn.sp_attn(lists, q, k, v, idx, cnt)
+    _capi().check()
+    _close(o, lists.cpu(), 8e-3, 5e-4)

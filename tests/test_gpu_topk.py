@@ -236,3 +236,44 @@ def test_topk_with_nan_scores(select_k):
     numbers = got[~bad[got]]
     want = torch.sort(torch.where(bad, torch.tensor(float("-inf")), x), descending=True, stable=True).indices
     assert torch.equal(numbers, want[: numbers.numel()])
+
+
+@pytest.mark.parametrize("kind", ["normal", "runs", "unlike_its_sample", "steps", "outlier", "nan"])
+@pytest.mark.parametrize("S,select_k", [(2000, 1), (3001, 300), (20000, 2000), (20001, 3900), (33000, 8192)])
+def test_topk_as_bits(kind, S, select_k):
+    """topk_packed sets the bits of the keys that topk_indices lists, whether the threshold comes from a sample of the row
+    (16 of every 128 bytes), from the general way because the sample was unlike the row, or from the sort."""
+    import fgattn_tk_cuda_b200.spattn  # noqa: F401  (registers torch.ops.cuda_attn)
+    capi = _capi()
+    g = torch.Generator().manual_seed(S + select_k)
+    B, H, rows, D = 1, 2, 300, 64
+    f = torch.randn(H, S, generator=g)
+    if kind == "runs":
+        f = 0.3 * f + 3 * torch.randn(H, S // 250 + 1, generator=g).repeat_interleave(250, 1)[:, :S]
+    elif kind == "unlike_its_sample":
+        f[:, torch.arange(S) % 32 < 4] += 20
+    elif kind == "steps":
+        f = torch.floor(2 * f)
+    elif kind == "outlier":
+        f[:, S // 3] = 3e4
+    elif kind == "nan":
+        f[:, S // 2] = float("nan")
+    q = torch.randn(B, H, rows, D, generator=g)
+    q[..., 0] = 2.0
+    k = 0.05 * torch.randn(B, H, S, D, generator=g)
+    k[0, :, :, 0] = f
+    q, k = q.to(torch.bfloat16).cuda(), k.to(torch.bfloat16).cuda()
+    stride = 128 * ((select_k + 127) // 128)
+    idx = torch.full((B, H, 3, stride), -1, dtype=torch.int32, device="cuda")
+    cnt = torch.full((B, H, 3), -1, dtype=torch.int32, device="cuda")
+    capi.topk_indices(idx, cnt, q, k, select_k, blocksz=128)
+    words = (S + 31) // 32 + 1
+    packed = torch.full((B, H, 3, 4 * words), 0xA5, dtype=torch.uint8, device="cuda")
+    torch.ops.cuda_attn.topk_packed(packed, q, k, select_k, 128)
+    capi.check()
+    want = torch.zeros(B * H * 3, 32 * words, dtype=torch.bool)
+    want.scatter_(1, idx.view(B * H * 3, stride)[:, :select_k].cpu().long(), True)
+    assert (want.sum(1) == select_k).all()
+    got = torch.zeros_like(want, dtype=torch.uint8).cuda()
+    capi.unpack_mask(got, packed.view(B * H * 3, 4 * words))
+    assert torch.equal(got.cpu().bool(), want)
