@@ -10,6 +10,7 @@
 // run on meta tensors without a GPU.
 #include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
+#include <nvtx3/nvToolsExt.h>
 #include <torch/extension.h>
 
 #include <map>
@@ -377,6 +378,42 @@ void sp_attn_blocks_ml(torch::Tensor o, torch::Tensor q, torch::Tensor k, torch:
                                         size_t(ws.numel()), stream_of(q)), "sp_attn_blocks_ml");
 }
 
+// block_index_lists and sp_attn_blocks_ml on its lists in one call, for sizes where launches and host time are what a
+// call costs: lists, max_q, denom, maxima and queue are one transient allocation.
+void attn_block_mask_check(torch::Tensor o, torch::Tensor q, torch::Tensor k, torch::Tensor v, double threshold) {
+  check_qk(q, k); check_v(v, k); check_o(o, q);
+  TORCH_CHECK(threshold > 0.0, "threshold must be positive");
+}
+void attn_block_mask(torch::Tensor o, torch::Tensor q, torch::Tensor k, torch::Tensor v, double threshold) {
+  attn_block_mask_check(o, q, k, v, threshold);
+  c10::cuda::CUDAGuard guard(q.device());
+  const int64_t B = q.size(0), H = q.size(1), S = q.size(2), K = k.size(2), D = q.size(3);
+  const int64_t nqb = cdiv(S, 64), nkb = cdiv(K, 64);
+  auto up = [](int64_t bytes) { return cdiv(bytes, 256) * 256; };
+  const int64_t b_idx = up(B * H * nqb * nkb * 4), b_cnt = up(B * H * nqb * 4), b_ml = up(B * H * pad128(S) * 4);
+  const int64_t b_max = int64_t(fgattn_block_scratch_bytes(int(B), int(H), int(S), int(K)));
+  const int64_t b_ws = int64_t(fgattn_sp_attn_workspace_bytes(int(B), int(H), int(S)));
+  torch::Tensor buf = torch::empty({b_idx + b_cnt + 2 * b_ml + up(b_max) + b_ws},
+                                   torch::TensorOptions().dtype(torch::kUInt8).device(q.device()));
+  char* at = static_cast<char*>(buf.data_ptr());
+  int* idx = reinterpret_cast<int*>(at);
+  int* cnt = reinterpret_cast<int*>(at + b_idx);
+  float* max_q = reinterpret_cast<float*>(at + b_idx + b_cnt);
+  float* denom = reinterpret_cast<float*>(at + b_idx + b_cnt + b_ml);
+  char* maxima = at + b_idx + b_cnt + 2 * b_ml;
+  void* const st = stream_of(q);
+  nvtxRangePushA("fgattn.maxq_denom+block_lists");
+  const int lists = fgattn_block_index_lists(idx, cnt, int(nkb), max_q, denom, nullptr, q.data_ptr(), k.data_ptr(), nullptr,
+                                             float(threshold), B, H, S, D, K, K, 0.f, maxima, size_t(b_max), st);
+  nvtxRangePop();
+  check_status(lists, "block_index_lists");
+  nvtxRangePushA("fgattn.sparse_attention");
+  const int attn = fgattn_sp_attn_blocks_ml(o.data_ptr(), q.data_ptr(), k.data_ptr(), v.data_ptr(), idx, cnt, int(nkb), max_q,
+                                            denom, B, H, S, D, K, K, 0.f, maxima + up(b_max), size_t(b_ws), st);
+  nvtxRangePop();
+  check_status(attn, "sp_attn_blocks_ml");
+}
+
 void sp_attn_blocks_hint_check(torch::Tensor o, torch::Tensor q, torch::Tensor k, torch::Tensor v,
                                torch::Tensor kb_indices, torch::Tensor kb_counts, torch::Tensor max_q_hint) {
   check_qk(q, k); check_v(v, k); check_o(o, q);
@@ -561,6 +598,7 @@ TORCH_LIBRARY_FRAGMENT(cuda_attn, m) {
   m.def("block_index_lists(Tensor (kb_indices!) kb_indices, Tensor (kb_counts!) kb_counts, Tensor (o_max_q!) o_max_q, Tensor (o_denom!) o_denom, Tensor(o!)? o, Tensor q, Tensor k, Tensor? v, float threshold, Tensor (scratch!) scratch) -> ()");
   m.def("block_lists_from_maxima(Tensor (kb_indices!) kb_indices, Tensor (kb_counts!) kb_counts, Tensor block_maxima, Tensor max_q, Tensor denom, int seq, int head_dim, int kv_seq_len, float threshold) -> ()");
   m.def("sp_attn_blocks_ml(Tensor (o!) o, Tensor q, Tensor k, Tensor v, Tensor kb_indices, Tensor kb_counts, Tensor max_q, Tensor denom) -> ()");
+  m.def("attn_block_mask(Tensor (o!) o, Tensor q, Tensor k, Tensor v, float threshold) -> ()");
   m.def("sp_attn_blocks(Tensor (o!) o, Tensor q, Tensor k, Tensor v, Tensor kb_indices, Tensor kb_counts) -> ()");
   m.def("sp_attn_blocks_hint(Tensor (o!) o, Tensor q, Tensor k, Tensor v, Tensor kb_indices, Tensor kb_counts, Tensor max_q_hint) -> ()");
   // one-bit-per-entry masks
@@ -590,6 +628,7 @@ TORCH_LIBRARY_IMPL(cuda_attn, Meta, m) {
   m.impl("block_index_lists", block_index_lists_check);
   m.impl("block_lists_from_maxima", block_lists_from_maxima_check);
   m.impl("sp_attn_blocks_ml", sp_attn_blocks_ml_check);
+  m.impl("attn_block_mask", attn_block_mask_check);
   m.impl("sp_attn_blocks", sp_attn_blocks_check);
   m.impl("sp_attn_blocks_hint", sp_attn_blocks_hint_check);
   m.impl("pack_mask", pack_mask_check);
@@ -615,6 +654,7 @@ TORCH_LIBRARY_IMPL(cuda_attn, CUDA, m) {
   m.impl("block_index_lists", block_index_lists);
   m.impl("block_lists_from_maxima", block_lists_from_maxima);
   m.impl("sp_attn_blocks_ml", sp_attn_blocks_ml);
+  m.impl("attn_block_mask", attn_block_mask);
   m.impl("sp_attn_blocks", sp_attn_blocks);
   m.impl("sp_attn_blocks_hint", sp_attn_blocks_hint);
   m.impl("pack_mask", pack_mask);

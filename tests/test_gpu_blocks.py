@@ -306,3 +306,18 @@ def test_lists_for_another_threshold_from_kept_maxima(S, D, kv):
         torch.ops.cuda_attn.block_lists_from_maxima(idx3, cnt3, scratch, m, l, S, D, n_kv, tau)
         assert torch.equal(cnt3, ref_cnt) and torch.equal(idx3, ref_idx)
     assert cnt2.sum().item() < cnt.sum().item()          # the higher threshold keeps fewer blocks
+
+
+@pytest.mark.parametrize("S,K,D", [(1, 1, 64), (64, 65, 128), (1024, 1024, 64), (777, 300, 128), (3000, 1111, 64)])
+def test_block_mask_step_in_one_operator(S, K, D):
+    """The step for small calls is one operator: bit for bit what the list build and the attention on its lists give."""
+    from fgattn_tk_cuda_b200 import capi, synth
+    from fgattn_tk_cuda_b200.spattn import mask_utils as mu, sparseattn_functionals as sf
+    w = synth.Workload("t", 2, 3, max(S, K), D, "clustered", centroids=10, run=80, tau=1e-3, seed=S + K)
+    q, k, v = synth.make_qkv(w, device="cuda")
+    q, k, v = q[:, :, :S], k[:, :, :K], v[:, :, :K]
+    assert q.numel() // D * K <= sf._ONE_CALL_PAIRS
+    o = sf.attn_computed_with_sparse_mask_cuda(q, k, v, thresh=w.tau, blocksz=64)
+    want = sf._sparse(sf._out(q), q, k, v, mu.qk_block_indexmask_cuda(q, k, w.tau))
+    capi.check()
+    assert torch.equal(o, want)
