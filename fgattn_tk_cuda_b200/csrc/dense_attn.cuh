@@ -17,8 +17,8 @@
 //                                                                  mode warp 9 alone)
 // S = Q K^T accumulates in tensor memory; the softmax warps read it with tcgen05.ld, write the
 // bf16 probabilities back over the same columns and the PV product takes them from tensor memory.
-// Tensor memory with V: S0 S1 O0 O1, 128 columns each; with rotating score buffers (ROT, at D = 64) three 128-column
-// ones that both tiles go round and two 64-column accumulators.  The output leaves through shared memory by TMA.
+// Tensor memory with V: S0 S1 O0 O1, 128 columns each; with rotating scores (ROT, at D = 64) 192 columns a tile that its
+// scores and probabilities rotate through and two 64-column accumulators.  The output leaves through shared memory by TMA.
 #pragma once
 #include "sm100_ptx.cuh"
 #include "softmax_steps.cuh"
@@ -78,7 +78,7 @@ enum : int {
   BAR_V_FULL = 9,    // +stage
   BAR_V_EMPTY = 13,  // +stage
   BAR_S_FULL = 17,   // +tile*2+buf
-  BAR_S_EMPTY = 21,  // +tile*2+buf
+  BAR_S_EMPTY = 21,  // +tile*2+buf (with rotating scores +tile*2+step parity: the step's scores are in registers)
   BAR_P_FULL = 25,   // +tile*2 (+step parity with rotating score buffers)
   BAR_O_FULL = 29,   // +tile
   BAR_PV_DONE = 31,  // +tile: rotating score buffers only, the tile's last P V product has been executed
@@ -96,13 +96,15 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   // without V the V ring's shared memory (it follows the K ring) holds K tiles as well
   constexpr int kKSt = HAS_V ? Cfg::kKStages : 4;
   static_assert(kKSt <= 4, "barrier slots");
-  // With V at D = 64 the accumulators take 64 columns each, which leaves room for a third score buffer.  The score
-  // tiles of both query tiles go round the three buffers (unit = step * tiles + tile, buffer = unit % 3): a tile's
-  // next scores are computed while its softmax warps are still busy with the current ones.  What is left in the chain of
-  // a step is the softmax itself, (2, 16, 4096, 64): 0.217 -> 0.207 ms; on clustered keys, where whole quarters are
-  // skipped and a step is shorter, (4, 24, 12345, 64) 4.99 -> 4.93 ms.  (The exponentials alone are 1536 clocks a step
-  // of both tiles, ex2 issuing once in 8 clocks a sub-partition, against 514 of products.)  The persistent form
-  // rotates where an item is long enough (kOneBufferMaxKeyTiles of the launcher).
+  // With V at D = 64 the accumulators take 64 columns each, which leaves every query tile 192 for its scores and
+  // probabilities.  The scores of step g are 128 columns from 64 (g mod 2) on, the probabilities 64 from 128 (g mod 2)
+  // on: next scores need the half of the present ones that the probabilities do not take, free as soon as they are in
+  // registers, and the place of the probabilities before.  So a step's scores are there when the softmax of the one
+  // before ends, and what is left in the chain is the softmax itself.  Against three
+  // 128-column buffers that both tiles went round, where a softmax warp waited 886 of 2680 clocks a step for its scores:
+  // (2, 16, 4096, 64) 212 -> 199 us, 24 heads of 8192 rows 598 -> 564, clustered keys at (4, 24, 12345, 64) 4.88 -> 4.52 ms;
+  // where the offset moves in most tiles (q and k of deviation 3) 238 -> 241 us.
+  // The persistent form rotates where an item is long enough (kOneBufferMaxKeyTiles of the launcher).
   static_assert(!ROT || (HAS_V && D == 64), "room for a third score buffer");
   constexpr uint32_t kColO = ROT ? 384 : 256, kOStride = ROT ? 64 : 128;
   constexpr bool TWO_ISS = (HAS_V && D == 128) || MODE == kML;   // one UMMA issuer warp per query tile ...
@@ -306,39 +308,43 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
       for (int item = first_item; item < p.n_items && ok; item += item_step, ++it, g0 += n_tiles) {
         ok = mbar_wait_warp(bar(BAR_Q_FULL), it & 1, ab, p.err, 201);
         if constexpr (ROT) {
-          // Units in order, round the buffers from item to item: the product Q K^T of unit v + n_t + 1 follows P V of
-          // unit v, whose probabilities lie in the buffer that it overwrites (two tiles) or at most a step behind (one
-          // tile; never more than two steps' scores are out, so no barrier of a step parity completes twice unseen).
-          // So the scores of step g are never published before P V of step g - 2 is done, which the softmax warps'
-          // wait for BAR_PV_DONE by the parity of step g - 1 relies on.
-          const int n_t = __popc(tiles), t0 = (tiles & 1u) ? 0 : 1, n_units = n_tiles * n_t;
-          auto qk_unit = [&](int v) {
-            const int jj = (n_t == 2) ? v >> 1 : v, ti = (n_t == 2) ? v & 1 : 0;
-            const uint32_t g = g0 + jj;
+          // The scores of step g + 1 are computed as soon as the softmax warps have those of step g in registers: they
+          // overwrite one half of the latter and the probabilities of step g - 1, whose product with V was issued before.
+          // So the scores of step g are never published before P V of step g - 2 is done, which the softmax warps' wait
+          // for BAR_PV_DONE by the parity of step g - 1 relies on.
+          const int t_last = (tiles & 2u) ? 1 : 0;
+          auto scores_of = [&](int j) {                    // of both tiles
+            const uint32_t g = g0 + j;
             const int ks = g % kKSt;
-            if (ti == 0) ok = mbar_wait_warp(bar(BAR_K_FULL + ks), (g / kKSt) & 1, ab, p.err, 202);
-            if (!ok) return;
-            tc_fence_after();
-            issue_qk(t0 + ti, ks, ((g0 * n_t + v) % 3) * 128);
-            umma_commit_elect(bar(BAR_S_FULL + (t0 + ti) * 2 + (g & 1)));
-            if (ti == n_t - 1) umma_commit_elect(bar(BAR_K_EMPTY + ks));
-            if (v == n_units - 1) umma_commit_elect(bar(BAR_Q_EMPTY));
+            ok = mbar_wait_warp(bar(BAR_K_FULL + ks), (g / kKSt) & 1, ab, p.err, 202);
+            for (int t = 0; t < 2 && ok; ++t) {
+              if (!((tiles >> t) & 1u)) continue;
+              if (j > 0) ok = mbar_wait_warp(bar(BAR_S_EMPTY + t * 2 + ((g - 1) & 1)), ((g - 1) >> 1) & 1, ab, p.err, 204);
+              if (!ok) break;
+              tc_fence_after();
+              issue_qk(t, ks, t * 192 + 64 * (g & 1));
+              umma_commit_elect(bar(BAR_S_FULL + t * 2 + (g & 1)));
+              if (t == t_last) umma_commit_elect(bar(BAR_K_EMPTY + ks));
+              if (t == t_last && j + 1 == n_tiles) umma_commit_elect(bar(BAR_Q_EMPTY));
+            }
           };
-          for (int v = 0; v < min(n_t + 1, n_units) && ok; ++v) qk_unit(v);
+          if (ok) scores_of(0);
 #pragma unroll 1
-          for (int v = 0; v < n_units && ok; ++v) {
-            const int jj = (n_t == 2) ? v >> 1 : v, ti = (n_t == 2) ? v & 1 : 0, t = t0 + ti;
-            const uint32_t g = g0 + jj;
+          for (int j = 0; j < n_tiles && ok; ++j) {
+            const uint32_t g = g0 + j;
             const int vs = g % Cfg::kVStages;
-            if (ti == 0) ok = mbar_wait_warp(bar(BAR_V_FULL + vs), (g / Cfg::kVStages) & 1, ab, p.err, 203);
-            if (ok) ok = mbar_wait_warp(bar(BAR_P_FULL + t * 2 + (g & 1)), (g >> 1) & 1, ab, p.err, 205);
-            if (!ok) break;
-            tc_fence_after();
-            issue_pv(t, vs, jj > 0, ((g0 * n_t + v) % 3) * 128);
-            umma_commit_elect(bar(BAR_PV_DONE + t));
-            if (ti == n_t - 1) umma_commit_elect(bar(BAR_V_EMPTY + vs));
-            if (jj == n_tiles - 1) umma_commit_elect(bar(BAR_O_FULL + t));
-            if (v + n_t + 1 < n_units) qk_unit(v + n_t + 1);
+            if (j + 1 < n_tiles) scores_of(j + 1);
+            if (ok) ok = mbar_wait_warp(bar(BAR_V_FULL + vs), (g / Cfg::kVStages) & 1, ab, p.err, 203);
+            for (int t = 0; t < 2 && ok; ++t) {
+              if (!((tiles >> t) & 1u)) continue;
+              ok = mbar_wait_warp(bar(BAR_P_FULL + t * 2 + (g & 1)), (g >> 1) & 1, ab, p.err, 205);
+              if (!ok) break;
+              tc_fence_after();
+              issue_pv(t, vs, j > 0, t * 192 + 128 * (g & 1));
+              umma_commit_elect(bar(BAR_PV_DONE + t));
+              if (t == t_last) umma_commit_elect(bar(BAR_V_EMPTY + vs));
+              if (j == n_tiles - 1) umma_commit_elect(bar(BAR_O_FULL + t));
+            }
           }
         } else if (HAS_V) {
           // P(t) lives over S(t) and the tensor pipe runs in order, so the first product of an item may
@@ -435,7 +441,7 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
         if (!ok) break;
         tc_fence_after();
         const uint32_t s_addr =
-            lane_base + (ROT ? ((tiles == 3u ? g * 2 + t : g) % 3) * 128 : HAS_V ? t * 128 : (t * 2 + b) * 128);
+            lane_base + (ROT ? t * 192 + 64 * b : HAS_V ? t * 128 : (t * 2 + b) * 128);
         const int key0 = tile_of(j) * 128;               // first key of this tile
         const int kv_left = p.kv_len - key0;             // valid keys in this tile
         const int valid0 = min(64, kv_left), valid1 = max(0, min(64, kv_left - 64));
@@ -492,10 +498,19 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
           }
         };
         const uint32_t o_addr = lane_base + kColO + t * kOStride;
-        if (ROT && j > 0 && kv_left >= 128)     // every tile but the first and a ragged last one
-          softmax_steady_step<D>(s_addr, s_addr, o_addr, c, st, mx0, mx1, quiet);
-        else
+        if constexpr (ROT) {
+          const uint32_t p_addr = lane_base + t * 192 + 128 * b;
+          auto loaded = [&]() {                            // the next step's scores may come
+            tc_fence_before();
+            mbar_arrive(bar(BAR_S_EMPTY + t * 2 + b));
+          };
+          if (j > 0 && kv_left >= 128)                     // every tile but the first and a ragged last one
+            softmax_steady_step<D>(s_addr, p_addr, o_addr, c, st, mx0, mx1, quiet, loaded, b != 0);
+          else
+            softmax_online_step<D, HAS_V>(s_addr, p_addr, o_addr, valid0, valid1, c, j == 0, st, mx0, mx1, nullptr, quiet, loaded);
+        } else {
           softmax_online_step<D, HAS_V>(s_addr, s_addr, o_addr, valid0, valid1, c, j == 0, st, mx0, mx1, nullptr, quiet);
+        }
         if (ROT && !ok) break;
         tc_fence_before();
         if (HAS_V) mbar_arrive(bar(BAR_P_FULL + t * 2 + (ROT ? g & 1 : 0)));

@@ -162,9 +162,9 @@ int launch_dense_k(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorM
 }
 
 constexpr int kPersistMaxKeyTiles = 8;     // persistent CTAs up to 1024 keys
-// Persistent CTAs at D = 64: the score buffers rotate above 512 keys.  16384 rows of 24 heads, one buffer a tile against
-// rotating ones: 77 keys 40.7 / 41.7 us, 128 keys 37.1 / 39.2, 512 keys level, 1000 keys 170.7 / 166.7
-constexpr int kOneBufferMaxKeyTiles = 4;
+// Persistent CTAs at D = 64: the scores rotate above 256 keys.  One buffer a tile against rotating scores: 16384 rows of
+// 24 heads, 77 keys level, 256 keys 55.4 / 56.4 us; 32768 rows of 40 heads, 512 keys 275 / 262 us
+constexpr int kOneBufferMaxKeyTiles = 2;
 // The max / denominator pass alone stays persistent up to 2048 keys: measured against its one-item kernel
 // (maxq_pass.cuh) at 32768 queries x 40 heads, D = 128 / 64: 1280 keys 16 / 12 % faster, 1536 keys 13 / 6 %,
 // 2048 keys 10 / 4 %, 3072 keys level / 1 % slower

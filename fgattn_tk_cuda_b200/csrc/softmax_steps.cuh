@@ -50,18 +50,20 @@ __device__ __forceinline__ void rescale_accumulator(uint32_t o_addr, float alpha
 //            2 %), 3 of 8 for the max / denominator pass (C3 2.49 -> 2.38 ms, C4 3.94 -> 3.45 ms); 4 of 8 is
 //            slower again: the polynomial costs ten issue slots per pair against two
 //   quiet  : called before the accumulator is touched (waits for a product that may still be adding to it)
+//   loaded : called when the scores are in registers
 struct NoWait {
   __device__ __forceinline__ void operator()() const {}
 };
-template <int D, bool WRITE_P, int POLY = (WRITE_P ? 2 : 3), class Quiet = NoWait>
+template <int D, bool WRITE_P, int POLY = (WRITE_P ? 2 : 3), class Quiet = NoWait, class Loaded = NoWait>
 __device__ __forceinline__ void softmax_online_step(uint32_t s_addr, uint32_t p_addr, uint32_t o_addr, int valid0,
                                                     int valid1, float c, bool first, OnlineState& st, float& mx0,
                                                     float& mx1, const uint32_t* colmask = nullptr,
-                                                    Quiet quiet = Quiet()) {
+                                                    Quiet quiet = Quiet(), Loaded loaded = Loaded()) {
   uint32_t r[128];
 #pragma unroll
   for (int cc = 0; cc < 4; ++cc) tmem_ld32(s_addr + cc * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[cc * 32]));
   tmem_ld_wait();
+  loaded();
   if (valid0 < 64 || valid1 < 64) {
 #pragma unroll
     for (int i = 0; i < 64; ++i) {
@@ -194,24 +196,29 @@ __device__ __forceinline__ void quarter_probs(uint32_t (&r)[32], float qmax, flo
 // offset in use may lag the running maximum by up to 2^8, so on most inputs it hardly ever moves: the exponentials start
 // against the offset as it stands, before the tile's maximum is known and while three quarters of the scores are still on
 // their way from tensor memory.  Where some row of the warp turns out to need a larger offset, nothing has been
-// written yet: the scores are loaded again and the probabilities of all quarters taken against the new one.  The results
-// are those of softmax_online_step bit for bit.  Taken at D = 64, where the softmax bounds a step: (2, 16, 4096, 64),
+// written yet: that first quarter is loaded again and the probabilities of all quarters taken against the new one.  The
+// results are those of softmax_online_step bit for bit (backwards the row sums add up in another order).  Taken at D = 64, where the softmax bounds a step: (2, 16, 4096, 64),
 // i.i.d. normal q and k, 0.224 -> 0.217 ms.  With scores so far apart that the offset moves in most tiles (deviation of
-// q and k 2 / 3 / 6) softmax_online_step alone takes 0.232 / 0.239 / 0.241 ms, this with the rotating score buffers of
-// the dense kernel 0.225 / 0.239 / 0.247 (0.244 / 0.265 / 0.272 when a tile was done over from its maximum on).
+// q and k 2 / 3 / 6) softmax_online_step alone takes 0.232 / 0.239 / 0.241 ms, this with the rotating score buffers that
+// the dense kernel had then 0.225 / 0.239 / 0.247 (0.244 / 0.265 / 0.272 when a tile was done over from its maximum on).
 // At D = 128 it is level to 2.5 % slower (32768 x 512 keys 0.374 -> 0.384 ms): there the two products and the hand-offs
 // pace a step.
-template <int D, int POLY = 2, class Quiet = NoWait>
+// `backwards` (warp-uniform): the quarters are taken last to first.  Only the first one taken is ever loaded again, so the
+// columns of the other half of the tile may be overwritten as soon as `loaded` has been called.
+template <int D, int POLY = 2, class Quiet = NoWait, class Loaded = NoWait>
 __device__ __forceinline__ void softmax_steady_step(uint32_t s_addr, uint32_t p_addr, uint32_t o_addr, float c,
-                                                    OnlineState& st, float& mx0, float& mx1, Quiet quiet = Quiet()) {
+                                                    OnlineState& st, float& mx0, float& mx1, Quiet quiet = Quiet(),
+                                                    Loaded loaded = Loaded(), bool backwards = false) {
   uint32_t r[4][32];
   float qm[4];
   const float neg_m = -st.m_used;
   uint64_t sum2 = f2_pack(0.f, 0.f);
-  tmem_ld32(s_addr, r[0]);
+  const uint32_t s_first = s_addr + (backwards ? 96 : 0), p_first = p_addr + (backwards ? 48 : 0);
+  const int ds = backwards ? -32 : 32, dp = backwards ? -16 : 16;
+  tmem_ld32(s_first, r[0]);
   tmem_ld_wait_for(r[0]);
 #pragma unroll
-  for (int w = 1; w < 4; ++w) tmem_ld32(s_addr + w * 32, r[w]);
+  for (int w = 1; w < 4; ++w) tmem_ld32(s_first + w * ds, r[w]);
   qm[0] = quarter_max(r[0]);
   quarter_probs<POLY>(r[0], qm[0], c, neg_m, sum2);
 #pragma unroll
@@ -219,15 +226,17 @@ __device__ __forceinline__ void softmax_steady_step(uint32_t s_addr, uint32_t p_
     tmem_ld_wait_for(r[w]);
     qm[w] = quarter_max(r[w]);
   }
-  mx0 = fmaxf(qm[0], qm[1]);
-  mx1 = fmaxf(qm[2], qm[3]);
+  loaded();
+  const float lo = fmaxf(qm[0], qm[1]), hi = fmaxf(qm[2], qm[3]);
+  mx0 = backwards ? hi : lo;
+  mx1 = backwards ? lo : hi;
   const float mx = fmaxf(mx0, mx1);
   st.m_true = fmaxf(st.m_true, mx);
   auto finish = [&](float off, int from) {
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
       if (w >= from) quarter_probs<POLY>(r[w], qm[w], c, off, sum2);
-      tmem_st16(p_addr + w * 16, *reinterpret_cast<uint32_t(*)[16]>(&r[w][0]));
+      tmem_st16(p_first + w * dp, *reinterpret_cast<uint32_t(*)[16]>(&r[w][0]));
     }
     float sum0, sum1;
     f2_unpack(sum2, sum0, sum1);
@@ -242,10 +251,8 @@ __device__ __forceinline__ void softmax_steady_step(uint32_t s_addr, uint32_t p_
     st.l *= alpha;
     quiet();
     rescale_accumulator<D>(o_addr, alpha);
-#pragma unroll
-    for (int w = 0; w < 4; ++w) tmem_ld32(s_addr + w * 32, r[w]);
-#pragma unroll
-    for (int w = 0; w < 4; ++w) tmem_ld_wait_for(r[w]);
+    tmem_ld32(s_first, r[0]);
+    tmem_ld_wait_for(r[0]);
     sum2 = f2_pack(0.f, 0.f);
     finish(-st.m_used, 0);
     return;
