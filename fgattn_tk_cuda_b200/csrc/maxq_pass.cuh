@@ -62,10 +62,15 @@ enum : int {
 
 // One 64-column share of a score tile: the thread's running (m, l) takes in its row's 64 scores at s_addr,
 // of which the first `valid` are live (warp-uniform).  mx returns their raw maximum.  POLY as in
-// softmax_online_step: of every eight pairs of columns, how many take the FMA-pipe exponential.
-template <int POLY>
-__device__ __forceinline__ void maxq_step64(uint32_t s_addr, int valid, float c, OnlineState& st, float& mx) {
+// softmax_online_step: of every eight pairs of columns, how many take the FMA-pipe exponential.  loaded() is called when
+// the scores are in registers: the buffer is free from there on, and the next product into it waits for the slowest of
+// the eight warps that read it (a warp waited 276 of 1550 clocks a step for its scores when buffers were given back after
+// the exponentials).  With the three-input maximum, 32 instructions fewer: lists of 96 heads of 12345 rows, D = 64 3.541 ->
+// 3.432 ms, of 32 heads of 16384, D = 128 2.033 -> 2.007 ms.
+template <int POLY, class Loaded>
+__device__ __forceinline__ void maxq_step64(uint32_t s_addr, int valid, float c, OnlineState& st, float& mx, Loaded loaded) {
   if (valid <= 0) {
+    loaded();
     mx = -INFINITY;
     return;
   }
@@ -73,21 +78,14 @@ __device__ __forceinline__ void maxq_step64(uint32_t s_addr, int valid, float c,
   tmem_ld32(s_addr, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
   tmem_ld32(s_addr + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
   tmem_ld_wait();
+  loaded();
   if (valid < 64) {
 #pragma unroll
     for (int i = 0; i < 64; ++i)
       if (i >= valid) r[i] = __float_as_uint(-INFINITY);
   }
-  // maxima of the two 32-column quarters, two chains each
-  float ch[4];
-#pragma unroll
-  for (int w = 0; w < 4; ++w) ch[w] = __uint_as_float(r[w * 16]);
-#pragma unroll
-  for (int i = 1; i < 16; ++i) {
-#pragma unroll
-    for (int w = 0; w < 4; ++w) ch[w] = fmaxf(ch[w], __uint_as_float(r[w * 16 + i]));
-  }
-  const float qmax[2] = {fmaxf(ch[0], ch[1]), fmaxf(ch[2], ch[3])};
+  const float qmax[2] = {quarter_max(*reinterpret_cast<uint32_t(*)[32]>(&r[0])),
+                         quarter_max(*reinterpret_cast<uint32_t(*)[32]>(&r[32]))};
   mx = fmaxf(qmax[0], qmax[1]);
   st.m_true = fmaxf(st.m_true, mx);
   const float ms = mx * c;
@@ -289,9 +287,10 @@ maxq_pass_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
         tc_fence_after();
         const int valid = min(64, p.kv_len - j * 128 - h * 64);
         float mx;
-        maxq_step64<Cfg::kPoly>(lane_base + (t * 2 + b) * 128 + h * 64, valid, c, st, mx);
-        tc_fence_before();
-        mbar_arrive(bar(MQ_S_EMPTY + t * 2 + b));
+        maxq_step64<Cfg::kPoly>(lane_base + (t * 2 + b) * 128 + h * 64, valid, c, st, mx, [&]() {
+          tc_fence_before();
+          mbar_arrive(bar(MQ_S_EMPTY + t * 2 + b));
+        });
         if (BLOCKMAX) {
           if (row < p.S_pad && j * 2 + h < p.nkb)
             p.blockmax[(size_t(bh) * p.nkb + size_t(j) * 2 + h) * p.S_pad + row] = mx;
