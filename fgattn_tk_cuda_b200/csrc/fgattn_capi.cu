@@ -592,7 +592,13 @@ int token_launch(fg::TokenParams& p, const CUtensorMap& mq, const CUtensorMap& m
     FG_CUDA(cudaGetLastError());
     p.order = ws + 4;
   }
-  dim3 grid(n_units * p.pairs, 1, 1);
+  // A less than half full last wave takes its items' query blocks apart (TokenParams::half_from), so that it takes about
+  // two thirds of an item's time: what paces one block is the chain of its own steps.  1536 items of equal length (top-k,
+  // 3276 of 32760 keys) on 148 SMs: 700 -> 684 us
+  const int n_items = n_units * p.pairs, rest = n_items % sms;
+  const bool cut = n_items > sms && rest > 0 && 2 * rest <= sms;
+  p.half_from = cut ? n_items - rest : n_items;
+  dim3 grid(p.half_from + (cut ? 2 * rest : 0), 1, 1);
   if (D == 128) {
     auto kern = fg::sparse_token_attn_kernel<128>;
     r = set_smem(kern, fg::TokenCfg<128>::kSmemBytes);

@@ -22,6 +22,9 @@ struct TokenParams {
   // 128-row query blocks
   const int* order;
   int pairs;
+  // Thread blocks from half_from on take one query block each: block half_from + 2 i + t the t-th of the item that block
+  // half_from + i would have.  The launcher cuts the items of a last wave that is less than half full, as the dense kernels'.
+  int half_from;
   // optional [BH, nqb]: query blocks with route != 0 are computed by the block-route kernel and are left
   // alone here (no loads, no stores)
   const int* route;
@@ -77,15 +80,17 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
   AbortState* ab = reinterpret_cast<AbortState*>(smem + Cfg::kOffBar + 8 * TB_COUNT + 8);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int item = p.order ? p.order[blockIdx.x] : int(blockIdx.x);
+  const int half = int(blockIdx.x) - p.half_from;        // >= 0: one query block of an item
+  const int place = half < 0 ? int(blockIdx.x) : p.half_from + (half >> 1);
+  const int item = p.order ? p.order[place] : place;
   const int bh = item / p.pairs;
   const int q0 = (item - bh * p.pairs) * 256;
-  bool skip[2] = {false, false};
+  bool skip[2] = {half >= 0 && (half & 1) != 0, half >= 0 && (half & 1) == 0};
   if (p.route) {
 #pragma unroll
     for (int t = 0; t < 2; ++t) {
       const int qb = (q0 >> 7) + t;
-      skip[t] = qb >= p.nqb || p.route[size_t(bh) * p.nqb + qb] != 0;
+      skip[t] |= qb >= p.nqb || p.route[size_t(bh) * p.nqb + qb] != 0;
     }
     if (skip[0] && skip[1]) return;                      // CTA-uniform, before any set-up
   }
@@ -118,12 +123,13 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
   // both slots are slot 0's, one K and one V tile for both: slot 1's list starts as if it held them too, what lies there
   // is the end of slot 0's.
   const int* lst;
-  int cnt0, cnt1, off1, n_c = 0;
+  int cnt0, cnt1, off1, n_c = 0, from1 = 0;              // from1: slot 1's steps before it are in slot 0's list
   if (p.split) {
     const int4 sp = p.split[item];
-    n_c = sp.x;
-    cnt0 = 128 * n_c + sp.y;
-    cnt1 = 128 * n_c + sp.z;
+    from1 = sp.x;
+    n_c = half < 0 ? sp.x : 0;                           // (one query block alone shares nothing)
+    cnt0 = skip[0] ? 0 : 128 * sp.x + sp.y;
+    cnt1 = skip[1] ? 0 : 128 * sp.x + sp.z;
     off1 = sp.y;
     lst = p.pair_lists + size_t(item) * p.pair_cap;
   } else {
@@ -170,7 +176,7 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
     int tok0 = 0, tok1 = 0, next0 = 0, next1 = 0;
     auto request = [&](int t, int j) {
       const int pos = j * 128 + row0 + lane;
-      const int a = (lane < nrows && pos < (t ? cnt1 : cnt0)) ? lst[(t ? off1 : 0) + pos] : 0;
+      const int a = (lane < nrows && pos < (t ? cnt1 : cnt0)) ? lst[(t && j >= from1 ? off1 : 0) + pos] : 0;
       if (t) next1 = a;
       else next0 = a;
     };
@@ -320,7 +326,7 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         const int pos = j * 128 + w * 32;
-        ahead[w] = (j >= n_c && pos + lane < c_mine) ? l_mine[pos] : j < n_c ? 0 : -1;      // (shared steps are full)
+        ahead[w] = (j >= from1 && pos + lane < c_mine) ? l_mine[pos] : j < from1 ? 0 : -1;      // (common steps are full)
       }
     };
     request(0);

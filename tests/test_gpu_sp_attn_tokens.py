@@ -308,3 +308,40 @@ def test_packed_mask_of_more_than_a_sweep():
     torch.ops.cuda_attn.sp_attn(lists, q, k, v, idx, cnt)
     _capi().check()
     _close(o, lists.cpu(), 8e-3, 5e-4)
+
+
+@pytest.mark.parametrize("D,S", [(128, 256), (64, 200)])
+def test_items_of_the_last_wave_in_halves(D, S):
+    """A few items more than SMs: the last ones are cut into their query blocks, one thread block each.  The same heads in
+    calls of at most an item per SM are not cut: the same bits from lists, the same within rounding from a packed mask
+    (a query block alone shares no tiles), rows of a block that keeps nothing and of one past the sequence included."""
+    import fgattn_tk_cuda_b200.spattn  # noqa: F401  (registers torch.ops.cuda_attn)
+    from fgattn_tk_cuda_b200.spattn import mask_utils as mu
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    H, n_kv, nb = sms + 7, 700, (S + 127) // 128
+    g = torch.Generator(device="cuda").manual_seed(S)
+    q = torch.randn(1, H, S, D, generator=g, device="cuda").to(torch.bfloat16)
+    k, v = (torch.randn(1, H, n_kv, D, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    bits = torch.rand(1, H, 1, 704, generator=g, device="cuda") < torch.rand(1, H, 1, 1, generator=g, device="cuda")
+    bits = (bits ^ (torch.rand(1, H, nb, 704, generator=g, device="cuda") < 0.1)).contiguous()
+    bits[0, sms + 2, 0] = False
+    packed = mu.pack(bits)
+    idx, cnt = mu.packedmask_to_indexmask_cuda(packed, n_kv)
+
+    def parts(op, *per_head):
+        out = torch.full_like(q, float("nan"))
+        for a, b in ((0, sms), (sms, H)):
+            o = torch.full_like(q[:, a:b], float("nan")).contiguous()
+            op(o, *(t[:, a:b].contiguous() for t in (q, k, v) + per_head))
+            out[:, a:b] = o
+        return out
+
+    o = torch.full_like(q, float("nan"))
+    torch.ops.cuda_attn.sp_attn(o, q, k, v, idx, cnt)
+    lists = parts(lambda *a: torch.ops.cuda_attn.sp_attn(*a), idx, cnt)
+    assert torch.equal(o, lists)
+    o2 = torch.full_like(q, float("nan"))
+    torch.ops.cuda_attn.sp_attn_packed(o2, q, k, v, packed, n_kv)
+    _close(o2, parts(lambda *a: torch.ops.cuda_attn.sp_attn_packed(*a, n_kv), packed).cpu(), 8e-3, 5e-4)
+    _close(o2, lists.cpu(), 8e-3, 5e-4)
+    _capi().check()
