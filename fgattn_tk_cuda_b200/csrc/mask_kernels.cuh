@@ -4,6 +4,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include "sm100_ptx.cuh"
+
 namespace fg {
 
 // ---------------------------------------------------------------------------------------------
@@ -25,6 +27,8 @@ block_threshold_compact_kernel(const float* __restrict__ blockmax, const float* 
   const int qb = blockIdx.x, bhl = blockIdx.y, bh = bh0 + bhl;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int r0 = qb * 64;
+  grid_trigger();
+  grid_wait();                         // for the pass, which may still be running (launch_behind)
   if (tid < 64) {
     const int row = r0 + tid;
     float t = INFINITY;

@@ -163,6 +163,7 @@ maxq_pass_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
+  if (BLOCKMAX) grid_trigger();        // the threshold kernel may come and wait
   const uint32_t tmem = *tmem_slot;
   const int n_tiles = p.n_kv_tiles;
 

@@ -43,6 +43,12 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
 }
 
+// Programmatic dependent launch.  A kernel launched behind another one with the attribute (launch_behind in the
+// launcher) may start when every thread block of that one has called grid_trigger or exited; nothing that earlier
+// kernels write is there before grid_wait has returned, and nothing that they still read may be written before it.
+__device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // ---------------------------------------------------------------------------------------------
 // mbarrier
 // ---------------------------------------------------------------------------------------------

@@ -238,6 +238,9 @@ sparse_ml_persistent_kernel(const __grid_constant__ CUtensorMap mq, const __grid
     for (int i = 0; i < 4; ++i) mbar_init(bar(PB_L_FULL + i), Cfg::kSmWarps);
     mbar_fence_init();
   }
+  // For the lists (launch_behind).  No tensor memory is taken before: a thread block of the kernel in front that is still to
+  // take its own on this SM would wait for this one.
+  grid_wait();
   if (warp == Cfg::kWarpProdK) {
     __syncwarp();
     tmem_alloc(smem_u32(tmem_slot), 512);
