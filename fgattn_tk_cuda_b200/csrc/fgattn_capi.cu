@@ -607,9 +607,9 @@ int token_launch(fg::TokenParams& p, const CUtensorMap& mq, const CUtensorMap& m
     const int n_groups = (n_units + group - 1) / group;
     group = (n_units + n_groups - 1) / n_groups;                      // groups of equal size
     int* ws = static_cast<int*>(workspace);
-    fg::sparse_order_kernel<<<(n_units + group - 1) / group, 1024, 0, st>>>(len, ws + 4, ws, len_rows, p.pairs, n_units,
-                                                                          group, subs, 1, shift);
-    FG_CUDA(cudaGetLastError());
+    r = launch_behind(fg::sparse_order_kernel, dim3((n_units + group - 1) / group), 1024, 0, st, len, ws + 4, ws, len_rows, p.pairs,
+                      n_units, group, subs, 1, shift, nullptr);
+    if (r) return r;
     p.order = ws + 4;
   }
   // A less than half full last wave takes its items' query blocks apart (TokenParams::half_from), so that it takes about
@@ -618,20 +618,13 @@ int token_launch(fg::TokenParams& p, const CUtensorMap& mq, const CUtensorMap& m
   const int n_items = n_units * p.pairs, rest = n_items % sms;
   const bool cut = n_items > sms && rest > 0 && 2 * rest <= sms;
   p.half_from = cut ? n_items - rest : n_items;
-  dim3 grid(p.half_from + (cut ? 2 * rest : 0), 1, 1);
-  if (D == 128) {
-    auto kern = fg::sparse_token_attn_kernel<128>;
-    r = set_smem(kern, fg::TokenCfg<128>::kSmemBytes);
-    if (r) return r;
-    kern<<<grid, fg::TokenCfg<128>::kThreads, fg::TokenCfg<128>::kSmemBytes, st>>>(mq, mo, p);
-  } else {
-    auto kern = fg::sparse_token_attn_kernel<64>;
-    r = set_smem(kern, fg::TokenCfg<64>::kSmemBytes);
-    if (r) return r;
-    kern<<<grid, fg::TokenCfg<64>::kThreads, fg::TokenCfg<64>::kSmemBytes, st>>>(mq, mo, p);
-  }
-  FG_CUDA(cudaGetLastError());
-  return FGATTN_OK;
+  const dim3 grid(p.half_from + (cut ? 2 * rest : 0));
+  auto go = [&](auto kern, int threads, int smem) -> int {
+    const int rr = set_smem(kern, smem);
+    return rr ? rr : launch_behind(kern, grid, threads, smem, st, mq, mo, p);
+  };
+  return D == 128 ? go(fg::sparse_token_attn_kernel<128>, fg::TokenCfg<128>::kThreads, fg::TokenCfg<128>::kSmemBytes)
+                  : go(fg::sparse_token_attn_kernel<64>, fg::TokenCfg<64>::kThreads, fg::TokenCfg<64>::kSmemBytes);
 }
 
 // Keys of one pair of query blocks: every key once and less than a tile of common ones twice.
@@ -742,10 +735,10 @@ int fgattn_sp_attn_packed(void* o, const void* q, const void* k, const void* v, 
   p.split = split;
   p.pair_lists = lists;
   p.pair_cap = packed_pair_cap(kv_rows);
-  fg::packed_pairs_kernel<<<dim3(p.pairs, n_units), 256, 0, st>>>(
-      packed, row_bytes, int(std::min<long long>(std::min(n_valid, kv_rows), 8LL * row_bytes)), p.nqb, p.pairs, p.pair_cap,
-      lists, split, cost);
-  FG_CUDA(cudaGetLastError());
+  r = launch_behind(fg::packed_pairs_kernel, dim3(p.pairs, n_units), 256, 0, st, packed, row_bytes,
+                    int(std::min<long long>(std::min(n_valid, kv_rows), 8LL * row_bytes)), p.nqb, p.pairs, p.pair_cap, lists, split,
+                    cost);
+  if (r) return r;
   return token_launch(p, mq, mo, n_units, D, kv_rows, workspace, cost, p.pairs, 1, 0, st);
 }
 
@@ -971,10 +964,10 @@ int launch_sparse_persistent(bool renorm, void* o, const void* q, const void* k,
     if (renorm) FG_CUDA(cudaMemsetAsync(p.redo, 0, size_t(p.n_items) * sizeof(int), st));
   } else {
     // an item is a pair of 64-row query blocks with one list each, or (token-derived lists) one 128-row block
-    fg::sparse_order_kernel<<<n_groups, 1024, 0, st>>>(
-        kb_counts, static_cast<int*>(workspace) + 4, p.queue, kb_mask ? p.npairs : p.nqb, p.npairs, n_units, group_heads,
-        1, kb_mask ? 1 : 2, 0, renorm ? p.redo : nullptr);
-    FG_CUDA(cudaGetLastError());
+    r = launch_behind(fg::sparse_order_kernel, dim3(n_groups), 1024, 0, st, kb_counts, static_cast<int*>(workspace) + 4, p.queue,
+                      kb_mask ? p.npairs : p.nqb, p.npairs, n_units, group_heads, 1, kb_mask ? 1 : 2, 0,
+                      renorm ? p.redo : nullptr);
+    if (r) return r;
   }
   const int grid = std::min(p.n_items, sms);
   const int smem = (D == 128) ? fg::SparseMLCfg<128>::smem_bytes(p.list_cap, p.nkb)
@@ -1164,14 +1157,16 @@ int topk_select(int* kv_indices, int* kv_num_indices, int list_stride, uint32_t*
     auto kern = fg::topk_scores_kernel<128>;
     r = set_smem(kern, fg::TopkScoreCfg<128>::kSmemBytes);
     if (r) return r;
-    kern<<<g_sc, fg::TopkScoreCfg<128>::kThreads, fg::TopkScoreCfg<128>::kSmemBytes, st>>>(m_hi, m_lo, mk, p);
+    r = launch_behind(kern, g_sc, fg::TopkScoreCfg<128>::kThreads, fg::TopkScoreCfg<128>::kSmemBytes, st, m_hi, m_lo, mk, p);
+    if (r) return r;
   } else {
     fg::qblock_mean_kernel<64><<<g_mean, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(q), qm_hi, qm_lo, seq, nblk,
                                                       blocksz, sc);
     auto kern = fg::topk_scores_kernel<64>;
     r = set_smem(kern, fg::TopkScoreCfg<64>::kSmemBytes);
     if (r) return r;
-    kern<<<g_sc, fg::TopkScoreCfg<64>::kThreads, fg::TopkScoreCfg<64>::kSmemBytes, st>>>(m_hi, m_lo, mk, p);
+    r = launch_behind(kern, g_sc, fg::TopkScoreCfg<64>::kThreads, fg::TopkScoreCfg<64>::kSmemBytes, st, m_hi, m_lo, mk, p);
+    if (r) return r;
   }
   FG_CUDA(cudaGetLastError());
   int k_pow2 = 2;
@@ -1182,10 +1177,8 @@ int topk_select(int* kv_indices, int* kv_num_indices, int list_stride, uint32_t*
   auto go = [&](auto kern) -> int {
     int rr = set_smem(kern, smem_sel);
     if (rr) return rr;
-    kern<<<unsigned(bh * nblk), fg::kSelThreads, smem_sel, st>>>(scores, s_stride, kv_seq_len, select_k, k_pow2, cap, kv_indices,
-                                                               kv_num_indices, list_stride, bits, row_bytes / 4);
-    FG_CUDA(cudaGetLastError());
-    return FGATTN_OK;
+    return launch_behind(kern, dim3(unsigned(bh * nblk)), fg::kSelThreads, smem_sel, st, scores, s_stride, kv_seq_len, select_k,
+                         k_pow2, cap, kv_indices, kv_num_indices, list_stride, bits, row_bytes / 4);
   };
   return bits ? go(fg::topk_select_kernel<true>) : go(fg::topk_select_kernel<false>);
 }

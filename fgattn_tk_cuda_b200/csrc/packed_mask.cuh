@@ -8,6 +8,7 @@
 #include <stdint.h>
 
 #include "mask_kernels.cuh"   // fill_tail
+#include "sm100_ptx.cuh"
 
 namespace fg {
 
@@ -211,6 +212,8 @@ packed_pairs_kernel(const uint8_t* __restrict__ packed, int row_bytes, int n_val
   static_assert(kChunks * kWarps == 32, "a lane per chunk and warp");
   __shared__ unsigned long long part[32];                // [chunk][warp]: common, first alone, second alone, 21 bits each
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  grid_trigger();
+  grid_wait();
   const int qb = 2 * blockIdx.x;
   const size_t item = size_t(blockIdx.y) * pairs + blockIdx.x;
   const uint8_t* src0 = packed + (size_t(blockIdx.y) * nqb + qb) * row_bytes;

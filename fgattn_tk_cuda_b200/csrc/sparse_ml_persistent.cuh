@@ -734,6 +734,8 @@ sparse_order_kernel(const int* __restrict__ kb_cnt, int* __restrict__ order, int
   __shared__ int hist[kBuckets];
   __shared__ int part[32];
   const int tid = threadIdx.x;
+  grid_trigger();
+  grid_wait();
   // the last group takes whatever is left (the launcher may make it larger than the others)
   const int u0 = blockIdx.x * group_heads, u1 = (blockIdx.x == gridDim.x - 1) ? n_units : min(n_units, u0 + group_heads);
   const int n = (u1 - u0) * npairs;

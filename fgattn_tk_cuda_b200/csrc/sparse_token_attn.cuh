@@ -80,6 +80,7 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
   AbortState* ab = reinterpret_cast<AbortState*>(smem + Cfg::kOffBar + 8 * TB_COUNT + 8);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  grid_wait();                                           // for lists and order (launch_behind)
   const int half = int(blockIdx.x) - p.half_from;        // >= 0: one query block of an item
   const int place = half < 0 ? int(blockIdx.x) : p.half_from + (half >> 1);
   const int item = p.order ? p.order[place] : place;

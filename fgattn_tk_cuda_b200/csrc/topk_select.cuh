@@ -27,6 +27,7 @@ qblock_mean_kernel(const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restric
   constexpr int kGroups = 256 / kChunks;         // row groups working in parallel
   __shared__ float part[kGroups][D];
   const int blk = blockIdx.x, bh = blockIdx.y, tid = threadIdx.x;
+  grid_trigger();
   const int chunk = tid % kChunks, grp = tid / kChunks;
   const int r0 = blk * blocksz, rows = min(blocksz, S - r0);
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
@@ -110,6 +111,8 @@ topk_scores_kernel(const __grid_constant__ CUtensorMap m_hi, const __grid_consta
     }
     mbar_fence_init();
   }
+  grid_trigger();
+  grid_wait();                         // for the means; before tensor memory is taken (launch_behind)
   if (warp == Cfg::kWarpProd) {
     __syncwarp();
     tmem_alloc(smem_u32(tmem_slot), 256);
@@ -276,6 +279,8 @@ topk_select_kernel(const float* __restrict__ scores, int s_stride, int n, int k,
   __shared__ uint32_t red_lo[kSelThreads / 32], red_hi[kSelThreads / 32];
   __shared__ int warp_tot[kSelThreads / 32];
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  grid_trigger();
+  grid_wait();
   const float* row = scores + size_t(blockIdx.x) * s_stride;
   const float4* row4 = reinterpret_cast<const float4*>(row);
   const int n4 = (n + 3) >> 2;
