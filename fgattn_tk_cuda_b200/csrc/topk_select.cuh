@@ -468,47 +468,64 @@ topk_select_kernel(const float* __restrict__ scores, int s_stride, int n, int k,
       if (s_rem < kSelBins) {
         const uint32_t from = float_order_key(f_hi - float(s_rem) / to_bin);
         uint32_t top = 0u;
-        for (int base = 0; base < n4; base += 4 * kSelThreads) {
-          float4 v[4];
+        // reach(x): the score counts.  A threshold above zero is compared as the integer that its bits are (the larger of two
+        // positive floats, NaN included, is the larger integer, and negative ones are negative integers): one instruction
+        // an entry where the order-preserving image takes four.
+        auto collect = [&](auto&& reach) {
+          for (int base = 0; base < n4; base += 4 * kSelThreads) {
+            float4 v[4];
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int j = base + u * kSelThreads + tid;
-            v[u] = (j < n4) ? row4[j] : make_float4(0.f, 0.f, 0.f, 0.f);
-          }
-          uint32_t take = 0u;
+            for (int u = 0; u < 4; ++u) {
+              const int j = base + u * kSelThreads + tid;
+              v[u] = (j < n4) ? row4[j] : make_float4(0.f, 0.f, 0.f, 0.f);
+            }
+            uint32_t take = 0u;
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const int j = base + u * kSelThreads + tid;
-            const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+            for (int u = 0; u < 4; ++u) {
+              const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
 #pragma unroll
-            for (int e = 0; e < 4; ++e)
-              if (float_order_key(x[e]) >= from && 4 * j + e < n) take |= 1u << (4 * u + e);
-          }
-          const int c = __popc(take);
-          int incl = c;
+              for (int e = 0; e < 4; ++e)
+                if (reach(x[e])) take |= 1u << (4 * u + e);
+            }
+            if (base + 4 * kSelThreads > n >> 2) {           // the row ends here: entries past it do not count
 #pragma unroll
-          for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, incl, o);
-            if (lane >= o) incl += t;
-          }
-          int at = 0;
-          if (lane == 31 && incl > 0) at = atomicAdd(&s_count, incl);
-          at = __shfl_sync(0xffffffffu, at, 31) + incl - c;
+              for (int u = 0; u < 4; ++u) {
+                const int left = n - 4 * (base + u * kSelThreads + tid);
+                if (left < 4) take &= ~((15u << (4 * u)) & (left <= 0 ? ~0u : ~((1u << (4 * u + left)) - 1u)));
+              }
+            }
+            const int c = __popc(take);
+            int incl = c;
 #pragma unroll
-          for (int u = 0; u < 4; ++u) {
-            const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+            for (int o = 1; o < 32; o <<= 1) {
+              const int t = __shfl_up_sync(0xffffffffu, incl, o);
+              if (lane >= o) incl += t;
+            }
+            int at = 0;
+            if (lane == 31 && incl > 0) at = atomicAdd(&s_count, incl);
+            at = __shfl_sync(0xffffffffu, at, 31) + incl - c;
 #pragma unroll
-            for (int e = 0; e < 4; ++e) {
-              if ((take >> (4 * u + e)) & 1u) {
-                const uint32_t key = float_order_key(x[e]);
-                top = max(top, key);
-                if (at < cap)
-                  sel[at] = (static_cast<unsigned long long>(key) << 32) |
-                            uint32_t(~uint32_t(4 * (base + u * kSelThreads + tid) + e));
-                ++at;
+            for (int u = 0; u < 4; ++u) {
+              const float x[4] = {v[u].x, v[u].y, v[u].z, v[u].w};
+#pragma unroll
+              for (int e = 0; e < 4; ++e) {
+                if ((take >> (4 * u + e)) & 1u) {
+                  const uint32_t key = float_order_key(x[e]);
+                  top = max(top, key);
+                  if (at < cap)
+                    sel[at] = (static_cast<unsigned long long>(key) << 32) |
+                              uint32_t(~uint32_t(4 * (base + u * kSelThreads + tid) + e));
+                  ++at;
+                }
               }
             }
           }
+        };
+        if (from > 0x80000000u) {
+          const int limit = int(from & 0x7fffffffu);
+          collect([&](float x) { return __float_as_int(x) >= limit; });
+        } else {
+          collect([&](float x) { return float_order_key(x) >= from; });
         }
         top = __reduce_max_sync(0xffffffffu, top);
         if (lane == 0) atomicMax(&s_max, top);
