@@ -120,6 +120,7 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   AbortState* ab = reinterpret_cast<AbortState*>(smem + Cfg::kOffBar + 8 * BAR_COUNT + 8);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  grid_wait();                         // before anything is read or tensor memory taken (launch_behind)
   int first_item = (MODE == kTokenMask && p.order) ? p.order[blockIdx.x] : int(blockIdx.x);
   const int item_step = gridDim.x;
   uint32_t tiles = 3u;                 // bit t: query tile t of the item is computed by this thread block

@@ -155,6 +155,7 @@ maxq_pass_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant__
     for (int t = 0; t < 2; ++t) mbar_init(bar(MQ_MERGE + t), 128);
     mbar_fence_init();
   }
+  grid_wait();                         // before tensor memory is taken (launch_behind)
   if (warp == Cfg::kWarpProd) {
     __syncwarp();
     tmem_alloc(smem_u32(tmem_slot), 512);
