@@ -134,8 +134,7 @@ int set_smem(K kernel, int bytes) {
 
 // A launch that may start while the kernel before it in the stream is still running its last thread blocks; the kernel
 // waits for it itself (grid_wait).  Worth the gap between two launches: 4 heads of 1024 rows, D = 64, mask and attention in
-// one operator 30.7 -> 26.6 us with
-// the kernels behind the first one, 24.2 with all; dense calls of 11 to 23 us 0.6 to 2.2 us less.
+// one operator 30.7 -> 26.6 us with the kernels behind the first one, 24.2 with all; dense calls of 11 to 23 us 0.6 to 2.2 us less.
 template <class... Params, class... Args>
 int launch_behind(void (*kern)(Params...), dim3 grid, int threads, int smem, cudaStream_t st, Args... args) {
   cudaLaunchAttribute attr;
@@ -342,8 +341,7 @@ int launch_sparse(void* o, const void* q, const void* k, const void* v, const in
   auto go = [&](auto kern) -> int {
     int rr = set_smem(kern, smem);
     if (rr) return rr;
-    kern<<<dim3(n_ctas, 1, 1), 384, smem, st>>>(mq, mk, mv, p);
-    return FGATTN_OK;
+    return launch_behind(kern, dim3(n_ctas), 384, smem, st, mq, mk, mv, p);
   };
   if (D == 128) r = redo ? go(fg::sparse_block_attn_kernel<128, true>) : go(fg::sparse_block_attn_kernel<128, false>);
   else r = redo ? go(fg::sparse_block_attn_kernel<64, true>) : go(fg::sparse_block_attn_kernel<64, false>);
@@ -1149,16 +1147,16 @@ int topk_select(int* kv_indices, int* kv_num_indices, int list_stride, uint32_t*
   if (r) return r;
   const dim3 g_mean(nblk, bh), g_sc(std::min(p.n_tiles, sms));
   if (D == 128) {
-    fg::qblock_mean_kernel<128><<<g_mean, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(q), qm_hi, qm_lo, seq, nblk,
-                                                       blocksz, sc);
+    r = launch_behind(fg::qblock_mean_kernel<128>, g_mean, 256, 0, st, static_cast<const __nv_bfloat16*>(q), qm_hi, qm_lo, seq, nblk, blocksz, sc);
+    if (r) return r;
     auto kern = fg::topk_scores_kernel<128>;
     r = set_smem(kern, fg::TopkScoreCfg<128>::kSmemBytes);
     if (r) return r;
     r = launch_behind(kern, g_sc, fg::TopkScoreCfg<128>::kThreads, fg::TopkScoreCfg<128>::kSmemBytes, st, m_hi, m_lo, mk, p);
     if (r) return r;
   } else {
-    fg::qblock_mean_kernel<64><<<g_mean, 256, 0, st>>>(static_cast<const __nv_bfloat16*>(q), qm_hi, qm_lo, seq, nblk,
-                                                      blocksz, sc);
+    r = launch_behind(fg::qblock_mean_kernel<64>, g_mean, 256, 0, st, static_cast<const __nv_bfloat16*>(q), qm_hi, qm_lo, seq, nblk, blocksz, sc);
+    if (r) return r;
     auto kern = fg::topk_scores_kernel<64>;
     r = set_smem(kern, fg::TopkScoreCfg<64>::kSmemBytes);
     if (r) return r;

@@ -82,6 +82,7 @@ sparse_block_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
   volatile int* n_union = reinterpret_cast<volatile int*>(smem + Cfg::kOffBar + 8 * SB_COUNT + 16);   // [2]
   uint32_t* lists = reinterpret_cast<uint32_t*>(smem + Cfg::kOffList);                                 // [2][cap]
   uint32_t* bitmaps = lists + 2 * p.list_cap;                                                          // [2][2][words]
+  grid_wait();                         // before anything is read or tensor memory taken (launch_behind)
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int words = (p.nkb + 31) / 32;

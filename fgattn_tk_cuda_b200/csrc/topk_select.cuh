@@ -28,6 +28,7 @@ qblock_mean_kernel(const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restric
   __shared__ float part[kGroups][D];
   const int blk = blockIdx.x, bh = blockIdx.y, tid = threadIdx.x;
   grid_trigger();
+  grid_wait();
   const int chunk = tid % kChunks, grp = tid / kChunks;
   const int r0 = blk * blocksz, rows = min(blocksz, S - r0);
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
