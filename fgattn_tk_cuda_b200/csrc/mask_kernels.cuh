@@ -17,8 +17,8 @@ namespace fg {
 // grid (nqb, heads_in_chunk), 256 threads; dynamic shared memory: 64 floats + nkb bytes.
 // ---------------------------------------------------------------------------------------------
 __global__ void __launch_bounds__(256)
-block_threshold_compact_kernel(const float* __restrict__ blockmax, const float* __restrict__ max_q,
-                               const float* __restrict__ denom, int* __restrict__ kb_idx, int* __restrict__ kb_cnt,
+block_threshold_compact_kernel(const float* blockmax, const float* max_q,
+                               const float* denom, int* kb_idx, int* kb_cnt,
                                int S, int S_pad, int nqb, int nkb, int list_stride, int bh0, float scale_log2,
                                float log2_tau) {
   extern __shared__ uint8_t sm[];

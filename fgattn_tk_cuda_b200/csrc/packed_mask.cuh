@@ -206,8 +206,8 @@ index_to_packed_kernel(const int* __restrict__ idx, const int* __restrict__ cnt,
 // over by a program, where finding the common keys is a pass of its own over them, it was level to 12 % slower.
 // grid (pairs, BH), 256 threads, 1024 words of either mask per sweep.  Counts travel three to a 64-bit word.
 __global__ void __launch_bounds__(256, 5)
-packed_pairs_kernel(const uint8_t* __restrict__ packed, int row_bytes, int n_valid, int nqb, int pairs, int cap,
-                    int* __restrict__ lists, int4* __restrict__ split, int* __restrict__ cost) {
+packed_pairs_kernel(const uint8_t* packed, int row_bytes, int n_valid, int nqb, int pairs, int cap,
+                    int* lists, int4* split, int* cost) {
   constexpr int kChunks = 4, kWarps = 8, kSweep = 256 * kChunks;
   static_assert(kChunks * kWarps == 32, "a lane per chunk and warp");
   __shared__ unsigned long long part[32];                // [chunk][warp]: common, first alone, second alone, 21 bits each

@@ -46,6 +46,8 @@ __device__ __forceinline__ void fence_proxy_async_smem() {
 // Programmatic dependent launch.  A kernel launched behind another one with the attribute (launch_behind in the
 // launcher) may start when every thread block of that one has called grid_trigger or exited; nothing that earlier
 // kernels write is there before grid_wait has returned, and nothing that they still read may be written before it.
+// So no parameter of such a kernel is __restrict__ and none is read through __ldg: both promise memory that does not change
+// while the kernel runs, and let a load be taken before the wait or from a cache that the wait does not clear.
 __device__ __forceinline__ void grid_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 

@@ -325,8 +325,8 @@ sparse_block_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
       const int valid1 = ((e1 >> (30 + half)) & 1u) ? min(64, p.kv_len - entry_kb(e1) * 64) : 0;
       uint32_t colmask[4] = {0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu};
       if (masks != nullptr) {
-        const unsigned long long m0 = valid0 > 0 ? __ldg(masks + 2 * j) : 0ull;
-        const unsigned long long m1 = valid1 > 0 ? __ldg(masks + 2 * j + 1) : 0ull;
+        const unsigned long long m0 = valid0 > 0 ? masks[2 * j] : 0ull;
+        const unsigned long long m1 = valid1 > 0 ? masks[2 * j + 1] : 0ull;
         colmask[0] = uint32_t(m0); colmask[1] = uint32_t(m0 >> 32);
         colmask[2] = uint32_t(m1); colmask[3] = uint32_t(m1 >> 32);
       }

@@ -633,7 +633,7 @@ sparse_ml_persistent_kernel(const __grid_constant__ CUtensorMap mq, const __grid
           const uint32_t e = list[2 * j + kb_sel];
           const int valid_kb = ((e >> (30 + half)) & 1u) ? min(64, p.kv_len - entry_kb(e) * 64) : 0;
           unsigned long long live64 = ~0ull;               // fetched before the wait for the scores
-          if (TOKEN && valid_kb > 0) live64 = __ldg(masks + 2 * j + kb_sel);
+          if (TOKEN && valid_kb > 0) live64 = masks[2 * j + kb_sel];
           const int sbuf = s % kSB;
           FG_TW(w_s, ok = mbar_wait(bar(PB_S_FULL + s % 6), (s / 6) & 1, ab, p.err, 1403));
           if (!ok) break;
@@ -727,9 +727,9 @@ sparse_ml_persistent_kernel(const __grid_constant__ CUtensorMap mq, const __grid
 // items takes 6 us, with 256 threads and a scan through shared memory it took 11).  Block 0 also clears the queue counter; with `redo`
 // every block clears the re-run flags of its items.
 __global__ void __launch_bounds__(1024)
-sparse_order_kernel(const int* __restrict__ kb_cnt, int* __restrict__ order, int* __restrict__ queue, int nqb,
+sparse_order_kernel(const int* kb_cnt, int* order, int* queue, int nqb,
                     int npairs, int n_units, int group_heads, int subs = 1, int elems = 2, int shift = 0,
-                    int* __restrict__ redo = nullptr) {
+                    int* redo = nullptr) {
   constexpr int kBuckets = 1024;
   __shared__ int hist[kBuckets];
   __shared__ int part[32];

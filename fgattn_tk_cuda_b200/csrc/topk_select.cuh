@@ -21,8 +21,8 @@ namespace fg {
 // grid (n_blocks, BH), 256 threads.
 template <int D>
 __global__ void __launch_bounds__(256)
-qblock_mean_kernel(const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ qm_hi,
-                   __nv_bfloat16* __restrict__ qm_lo, int S, int n_blocks, int blocksz, float scale) {
+qblock_mean_kernel(const __nv_bfloat16* q, __nv_bfloat16* qm_hi,
+                   __nv_bfloat16* qm_lo, int S, int n_blocks, int blocksz, float scale) {
   constexpr int kChunks = D / 8;                 // 16-byte chunks per row
   constexpr int kGroups = 256 / kChunks;         // row groups working in parallel
   __shared__ float part[kGroups][D];
@@ -270,8 +270,8 @@ inline int select_capacity(int k) {
 // 32760 scores, k = 3276: 0.449 -> 0.235 ms with bits (the general way and the counting of places, all rows).
 template <bool BITS>
 __global__ void __launch_bounds__(kSelThreads, 3)
-topk_select_kernel(const float* __restrict__ scores, int s_stride, int n, int k, int k_pow2, int cap, int* __restrict__ idx,
-                   int* __restrict__ cnt, int list_stride, uint32_t* __restrict__ bits, int row_words) {
+topk_select_kernel(const float* scores, int s_stride, int n, int k, int k_pow2, int cap, int* idx,
+                   int* cnt, int list_stride, uint32_t* bits, int row_words) {
   // (key << 32 | ~index), cap entries and room for a bin's; then cap slots, or the row's bits
   extern __shared__ unsigned long long sel[];
   __shared__ int hist[kSelBins];
