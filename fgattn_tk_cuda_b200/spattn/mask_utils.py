@@ -358,16 +358,3 @@ def qk_topkmask_indices(q, k, select_k, B=None, H=None, S=None, D=None, BLOCKSZ=
     spattn_interface.topk_indices(kv_indices, kv_num_indices, q.contiguous(), k.contiguous(), int(select_k),
                                   int(BLOCKSZ))
     return kv_indices, kv_num_indices
-
-
-# keys per row of a selection handed over as bits, which are put together in shared memory beside the selected entries
-MAX_PACKED_SELECTION = 524288
-
-
-def _qk_topk_packed(q, k, select_k, blocksz=128):
-    """The keys of qk_topkmask_indices as one bit per key (uint8, pad128(S_kv) / 8 bytes a row): for an attention step,
-    which does not ask in what order they were selected."""
-    B, H, S, _ = q.shape
-    packed = torch.empty((B, H, (S + blocksz - 1) // blocksz, _pad128(k.shape[2]) // 8), dtype=torch.uint8, device=q.device)
-    spattn_interface.topk_packed(packed, q.contiguous(), k.contiguous(), int(select_k), int(blocksz))
-    return packed

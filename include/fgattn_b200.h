@@ -306,7 +306,7 @@ int fgattn_topk_indices(int* kv_indices, int* kv_num_indices, int list_stride, c
                         float scale, void* scratch, size_t scratch_bytes, void* stream);
 
 /* The same selection as a packed mask (one bit per key, rows of row_bytes bytes, a multiple of 4 and at least
- * kv_seq_len / 8): what fgattn_sp_attn_packed takes.  packed [B,H,ceil(seq/blocksz),row_bytes], 4-byte aligned. */
+ * kv_seq_len / 8), for a program that asks for the set of keys and not for their order.  packed [B,H,ceil(seq/blocksz),row_bytes], 4-byte aligned. */
 int fgattn_topk_packed(unsigned char* packed, int row_bytes, const void* q, const void* k, int select_k, int batch, int heads,
                        int seq, int D, int blocksz, int kv_rows, int kv_seq_len, float scale, void* scratch,
                        size_t scratch_bytes, void* stream);

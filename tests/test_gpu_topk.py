@@ -277,3 +277,23 @@ def test_topk_as_bits(kind, S, select_k):
     got = torch.zeros_like(want, dtype=torch.uint8).cuda()
     capi.unpack_mask(got, packed.view(B * H * 3, 4 * words))
     assert torch.equal(got.cpu().bool(), want)
+
+
+@pytest.mark.parametrize("S,D,select_k", [(2000, 128, 200), (5001, 64, 600), (3000, 128, 1500)])
+def test_topk_attention_takes_keys_by_score(S, D, select_k):
+    """attn_topkmask_cuda attends to the keys in descending order of their scores, as topk_indices lists them: bit for bit
+    what sp_attn gives on those lists.  (Another order rounds the probability that weighs most: a larger error.)"""
+    from fgattn_tk_cuda_b200 import synth
+    from fgattn_tk_cuda_b200.spattn import mask_utils as mu, sparseattn_functionals as sf
+    q, k, v = synth.make_qkv(synth.Workload("t", 1, 3, S, D, "clustered", centroids=16, run=64, seed=S), device="cuda")
+    o = sf.attn_topkmask_cuda(q, k, v, select_k=select_k, blocksz=128)
+    idx, cnt = mu.qk_topkmask_indices(q, k, select_k)
+    want = torch.empty_like(o)
+    torch.ops.cuda_attn.sp_attn(want, q, k, v, idx, cnt)
+    # the same keys in ascending order are not the same bits, or this test would show nothing
+    by_key = torch.empty_like(o)
+    ascending = torch.cat([idx[..., :select_k].sort(-1).values, idx[..., select_k:]], -1).contiguous()
+    torch.ops.cuda_attn.sp_attn(by_key, q, k, v, ascending, cnt)
+    _capi().check()
+    assert torch.equal(o, want)
+    assert not torch.equal(by_key, want)
