@@ -169,7 +169,7 @@ void sp_attn(torch::Tensor o, torch::Tensor q, torch::Tensor k, torch::Tensor v,
 }
 
 // sp_attn on a packed mask instead of lists: uint8 [B,H,ceil(S/128),W/8], one bit per key, of which the first n_valid count.
-// The workspace holds the kept keys of every pair of query blocks, half of what lists would take; it is not kept.
+// The workspace holds the lists of the bits; it is not kept.
 void sp_attn_packed_check(torch::Tensor o, torch::Tensor q, torch::Tensor k, torch::Tensor v, torch::Tensor packed,
                           int64_t n_valid) {
   check_qk(q, k); check_v(v, k); check_o(o, q);

@@ -8,7 +8,6 @@
 #include <stdint.h>
 
 #include "mask_kernels.cuh"   // fill_tail
-#include "sm100_ptx.cuh"
 
 namespace fg {
 
@@ -189,118 +188,6 @@ index_to_packed_kernel(const int* __restrict__ idx, const int* __restrict__ cnt,
     for (int w = tid; w < n_words; w += 256) reinterpret_cast<uint32_t*>(dst)[w] = s_bits[w];
   } else {
     for (int b = tid; b < row_bytes; b += 256) dst[b] = uint8_t(s_bits[b >> 2] >> (8 * (b & 3)));
-  }
-}
-
-// Packed masks of two neighbouring query blocks -> what both keep, in whole tiles of 128 keys, and what is left of each.
-//
-// The token-list attention runs two 128-row query blocks per thread block, and what bounds it is the row gather: every
-// kept key's K and V row is fetched once for each of the two.  Neighbouring blocks keep much the same keys (rows of one
-// region of the sequence look at the same part of it), so the tiles of common keys are fetched once for both.  A block's
-// number of 128-key steps is what its own list would take: common keys past the last whole tile go to both remainders.
-// Per pair the list row of `cap` entries holds 128 x common keys, then the remainder of the first block (y keys), then that
-// of the second (z); split = (x, y, z, 0), cost = tiles to gather.  All three ascend.
-// 12 heads of 256 query blocks and 32760 keys, 5 % kept: 36 us, where the lists of all blocks took 45 (packed_to_index_kernel).
-// Entries put together in shared memory first, to leave as whole lines: 36 to 50 us (bank conflicts).  Sharing is worth
-// up to 7 % of the attention there, as long as what bounds a step is the chain of softmax and products: on lists handed
-// over by a program, where finding the common keys is a pass of its own over them, it was level to 12 % slower.
-// grid (pairs, BH), 256 threads, 1024 words of either mask per sweep.  Counts travel three to a 64-bit word.
-__global__ void __launch_bounds__(256, 5)
-packed_pairs_kernel(const uint8_t* packed, int row_bytes, int n_valid, int nqb, int pairs, int cap,
-                    int* lists, int4* split, int* cost) {
-  constexpr int kChunks = 4, kWarps = 8, kSweep = 256 * kChunks;
-  static_assert(kChunks * kWarps == 32, "a lane per chunk and warp");
-  __shared__ unsigned long long part[32];                // [chunk][warp]: common, first alone, second alone, 21 bits each
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  grid_trigger();
-  grid_wait();
-  const int qb = 2 * blockIdx.x;
-  const size_t item = size_t(blockIdx.y) * pairs + blockIdx.x;
-  const uint8_t* src0 = packed + (size_t(blockIdx.y) * nqb + qb) * row_bytes;
-  const bool two = qb + 1 < nqb, words = ((row_bytes & 3) == 0) && ((reinterpret_cast<uintptr_t>(src0) & 3) == 0);
-  const int n_words = min((row_bytes + 3) >> 2, (n_valid + 31) >> 5);
-  auto word_of = [&](const uint8_t* src, int w) -> uint32_t {
-    uint32_t u = 0;
-    if (words) {
-      u = reinterpret_cast<const uint32_t*>(src)[w];
-    } else {
-#pragma unroll
-      for (int e = 0; e < 4; ++e)
-        if (4 * w + e < row_bytes) u |= uint32_t(src[4 * w + e]) << (8 * e);
-    }
-    const int left = n_valid - 32 * w;
-    return left < 32 ? u & ((1u << left) - 1u) : u;      // (left > 0: w < n_words)
-  };
-  auto counts_of = [](uint32_t a, uint32_t b) -> unsigned long long {
-    return (unsigned long long)(__popc(a & b)) | (unsigned long long)(__popc(a & ~b)) << 21 |
-           (unsigned long long)(__popc(b & ~a)) << 42;
-  };
-  auto scan = [&](unsigned long long x) {                // inclusive, over the lanes
-#pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-      const unsigned long long t = __shfl_up_sync(0xffffffffu, x, o);
-      if (lane >= o) x += t;
-    }
-    return x;
-  };
-  auto field = [](unsigned long long x, int i) { return int(x >> (21 * i)) & 0x1fffff; };
-
-  unsigned long long base = 0, total = 0;                // entries of the sweeps before this one, and of all
-  if (n_words > kSweep) {
-    for (int w = tid; w < n_words; w += 256) total += counts_of(word_of(src0, w), two ? word_of(src0 + row_bytes, w) : 0u);
-    total = scan(total);
-    if (lane == 31) part[warp] = total;
-    __syncthreads();
-    total = 0;
-#pragma unroll
-    for (int w = 0; w < kWarps; ++w) total += part[w];
-    __syncthreads();
-  }
-  int* const out = lists + item * cap;
-  for (int w0 = 0; w0 < n_words || w0 == 0; w0 += kSweep) {
-    uint32_t a[kChunks], b[kChunks];
-    unsigned long long c[kChunks], incl[kChunks];
-#pragma unroll
-    for (int k = 0; k < kChunks; ++k) {
-      const int w = w0 + k * 256 + tid;
-      a[k] = w < n_words ? word_of(src0, w) : 0u;
-      b[k] = (w < n_words && two) ? word_of(src0 + row_bytes, w) : 0u;
-    }
-#pragma unroll
-    for (int k = 0; k < kChunks; ++k) {
-      c[k] = counts_of(a[k], b[k]);
-      incl[k] = scan(c[k]);
-      if (lane == 31) part[k * kWarps + warp] = incl[k];
-    }
-    __syncthreads();
-    const unsigned long long mine = part[lane], upto = scan(mine);
-    const unsigned long long sweep = __shfl_sync(0xffffffffu, upto, 31);
-    if (n_words <= kSweep) total = sweep;
-    const int tiles = field(total, 0) >> 7, whole = tiles << 7, rest = field(total, 0) & 127;
-    const int len0 = rest + field(total, 1), len1 = rest + field(total, 2);
-    int* const out1 = out + whole + len0;                // the second block's remainder
-    if (tid == 0 && w0 == 0) {
-      split[item] = make_int4(tiles, len0, len1, 0);
-      cost[item] = tiles + ((len0 + 127) >> 7) + ((len1 + 127) >> 7);
-    }
-#pragma unroll
-    for (int k = 0; k < kChunks; ++k) {
-      const unsigned long long at = base + __shfl_sync(0xffffffffu, upto - mine, k * kWarps + warp) + incl[k] - c[k];
-      const int first = w0 + k * 256 + warp * 32;
-      const int at0 = field(at, 0);
-      const uint32_t both = a[k] & b[k];
-      // the common keys, of which the last `rest` are where the first remainder starts, and once more in the second
-      write_entries(both, field(c[k], 0), at0, first, out, cap);
-      if (__any_sync(0xffffffffu, at0 + field(c[k], 0) > whole)) {
-        uint32_t u = both;
-        for (int e = at0; u; ++e, u &= u - 1)
-          if (e >= whole) out1[e - whole] = 32 * (first + lane) + __ffs(u) - 1;
-      }
-      write_entries(a[k] & ~b[k], field(c[k], 1), field(at, 1), first, out + field(total, 0), cap);
-      write_entries(b[k] & ~a[k], field(c[k], 2), field(at, 2), first, out1 + rest, cap);
-    }
-    base += sweep;
-    __syncthreads();                                     // `part` is free for the next sweep
   }
 }
 

@@ -28,11 +28,6 @@ struct TokenParams {
   // optional [BH, nqb]: query blocks with route != 0 are computed by the block-route kernel and are left
   // alone here (no loads, no stores)
   const int* route;
-  // optional, instead of kv_idx and kv_cnt: per item (tiles of 128 keys that both query blocks keep, keys left of the first,
-  // keys left of the second), their keys in this order in pair_lists[item * pair_cap ..) (packed_pairs_kernel)
-  const int4* split;
-  const int* pair_lists;
-  int pair_cap;
   float scale_log2;
 };
 
@@ -120,30 +115,14 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
 
-  // Per-slot list length and number of 128-token steps; slot t's list starts at lst + t * off1.  The first n_c steps of
-  // both slots are slot 0's, one K and one V tile for both: slot 1's list starts as if it held them too, what lies there
-  // is the end of slot 0's.
-  const int* lst;
-  int cnt0, cnt1, off1, n_c = 0, from1 = 0;              // from1: slot 1's steps before it are in slot 0's list
-  if (p.split) {
-    const int4 sp = p.split[item];
-    from1 = sp.x;
-    n_c = half < 0 ? sp.x : 0;                           // (one query block alone shares nothing)
-    cnt0 = skip[0] ? 0 : 128 * sp.x + sp.y;
-    cnt1 = skip[1] ? 0 : 128 * sp.x + sp.z;
-    off1 = sp.y;
-    lst = p.pair_lists + size_t(item) * p.pair_cap;
-  } else {
-    auto list_length = [&](int t) {
-      const int qb = (q0 >> 7) + t;
-      const bool none = qb >= p.nqb || (t ? skip[1] : skip[0]);
-      return none ? 0 : max(0, min(p.kv_cnt[size_t(bh) * p.nqb + qb], p.mask_stride));
-    };
-    cnt0 = list_length(0);
-    cnt1 = list_length(1);
-    off1 = p.mask_stride;
-    lst = p.kv_idx + (size_t(bh) * p.nqb + (q0 >> 7)) * p.mask_stride;
-  }
+  // per-slot list length and number of 128-token steps; slot t's list starts at lst + t * mask_stride
+  auto list_length = [&](int t) {
+    const int qb = (q0 >> 7) + t;
+    const bool none = qb >= p.nqb || (t ? skip[1] : skip[0]);
+    return none ? 0 : max(0, min(p.kv_cnt[size_t(bh) * p.nqb + qb], p.mask_stride));
+  };
+  const int cnt0 = list_length(0), cnt1 = list_length(1);
+  const int* const lst = p.kv_idx + (size_t(bh) * p.nqb + (q0 >> 7)) * p.mask_stride;
   const int nst0 = (cnt0 + 127) >> 7, nst1 = (cnt1 + 127) >> 7, n_max = max(nst0, nst1);
 
   if (warp == 8 || warp >= 10) {
@@ -177,7 +156,7 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
     int tok0 = 0, tok1 = 0, next0 = 0, next1 = 0;
     auto request = [&](int t, int j) {
       const int pos = j * 128 + row0 + lane;
-      const int a = (lane < nrows && pos < (t ? cnt1 : cnt0)) ? lst[(t && j >= from1 ? off1 : 0) + pos] : 0;
+      const int a = (lane < nrows && pos < (t ? cnt1 : cnt0)) ? lst[(t ? p.mask_stride : 0) + pos] : 0;
       if (t) next1 = a;
       else next0 = a;
     };
@@ -189,7 +168,7 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
       request(t, j + 1);
     };
     request(0, 0);
-    request(1, n_c);
+    request(1, 0);
     // Each copy instruction moves whole rows: 16 (D = 128) or 8 (D = 64) neighbouring lanes fetch the
     // consecutive 16-byte chunks of one row, so a warp-wide copy asks L2 for full 128-byte lines
     // instead of 32 separate sectors.
@@ -213,14 +192,10 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
       pending_stage = st;
       ++idx;
     };
-    // Order: K(0,0) K(1,0), then per step V(t,j) K(t,j+1); the ids of step j serve K(t,j) and V(t,j).  With shared steps
-    // K(0), then for each of them V(j) and K(j+1), after the last one K(0,n_c) K(1,n_c).
-    for (int j = 0; j <= n_c && ok; ++j) {
-      if (j > 0) gather_tile(p.v, 0);
-      if (ok && j < nst0) { take_tokens(0, j); gather_tile(p.k, 0); }
-    }
-    if (n_c < nst1 && ok) { take_tokens(1, n_c); gather_tile(p.k, 1); }
-    for (int j = n_c; j < n_max && ok; ++j) {
+    // order: K(0,0) K(1,0), then per step V(t,j) K(t,j+1); the ids of step j serve K(t,j) and V(t,j)
+    if (nst0 > 0) { take_tokens(0, 0); gather_tile(p.k, 0); }
+    if (nst1 > 0 && ok) { take_tokens(1, 0); gather_tile(p.k, 1); }
+    for (int j = 0; j < n_max && ok; ++j) {
 #pragma unroll
       for (int t = 0; t < 2; ++t) {
         const int n = t ? nst1 : nst0;
@@ -247,10 +222,9 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
       const uint32_t idesc_pv = umma_idesc_bf16(128, D, true);
       int idx = 0;
       bool ok = mbar_wait_warp(bar(TB_Q_FULL), 0, ab, p.err, 801);
-      // tile `at` of the ring; `done`: this is its last product
-      auto qk = [&](int t, int at, bool done) {
-        const int st = at % Cfg::kStages;
-        ok = mbar_wait_warp(bar(TB_FULL + st), (at / Cfg::kStages) & 1, ab, p.err, 802);
+      auto qk = [&](int t) {
+        const int st = idx % Cfg::kStages;
+        ok = mbar_wait_warp(bar(TB_FULL + st), (idx / Cfg::kStages) & 1, ab, p.err, 802);
         if (!ok) return;
         tc_fence_after();
         const uint32_t qa = sbase + Cfg::kOffQ + t * Cfg::kTileBytes, ka = sbase + Cfg::kOffRing + st * Cfg::kTileBytes;
@@ -262,13 +236,14 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
                     idesc_qk, ks > 0);
           }
           umma_commit(bar(TB_S_FULL + t));
-          if (done) umma_commit(bar(TB_EMPTY + st));
+          umma_commit(bar(TB_EMPTY + st));
         }
         __syncwarp();
+        ++idx;
       };
-      auto pv = [&](int t, int j, int at, bool done) {
-        const int st = at % Cfg::kStages;
-        ok = mbar_wait_warp(bar(TB_FULL + st), (at / Cfg::kStages) & 1, ab, p.err, 803);
+      auto pv = [&](int t, int j) {
+        const int st = idx % Cfg::kStages;
+        ok = mbar_wait_warp(bar(TB_FULL + st), (idx / Cfg::kStages) & 1, ab, p.err, 803);
         if (ok) ok = mbar_wait_warp(bar(TB_P_FULL + t), j & 1, ab, p.err, 804);
         if (!ok) return;
         tc_fence_after();
@@ -278,32 +253,22 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
           for (int ks = 0; ks < 8; ++ks)
             umma_ts(tmem + 256 + t * 128, tmem + t * 128 + ks * 8, umma_smem_desc_sw128(va + ks * 2048, 16384, 1024),
                     idesc_pv, (j > 0 || ks > 0) ? 1u : 0u);
-          if (done) umma_commit(bar(TB_EMPTY + st));
+          umma_commit(bar(TB_EMPTY + st));
         }
         __syncwarp();
+        ++idx;
       };
       // the tiles in the order of the gather warps
-      for (int t = 0; t < 2 && ok; ++t)
-        if ((t ? nst1 : nst0) > 0) {
-          qk(t, idx, n_c == 0 || t == 1);
-          if (n_c == 0 || t == 1) ++idx;
-        }
+      if (ok && nst0 > 0) qk(0);
+      if (ok && nst1 > 0) qk(1);
       for (int j = 0; j < n_max && ok; ++j) {
-        const bool one_v = j < n_c, one_k = j + 1 < n_c;   // this step's V tile, the next step's K tile serves both slots
-        int at_v = idx;
-        if (one_v) ++idx;
         for (int t = 0; t < 2 && ok; ++t) {
           const int n = t ? nst1 : nst0;
           if (j < n) {
-            if (!one_v) at_v = idx++;
-            pv(t, j, at_v, !one_v || t == 1);
+            pv(t, j);
             if (!ok) break;
-            if (j + 1 < n) {
-              qk(t, idx, !one_k || t == 1);
-              if (!one_k || t == 1) ++idx;
-            } else {
-              umma_commit_elect(bar(TB_O_FULL + t));
-            }
+            if (j + 1 < n) qk(t);
+            else umma_commit_elect(bar(TB_O_FULL + t));
           }
         }
       }
@@ -321,13 +286,13 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
     // Which of a step's 128 gathered columns are real keys: the entries are requested when the step before has been
     // computed and looked at when the step's scores are there.
     const int n_mine = t ? nst1 : nst0, c_mine = t ? cnt1 : cnt0;
-    const int* const l_mine = lst + (t ? off1 : 0) + lane;
+    const int* const l_mine = lst + (t ? p.mask_stride : 0) + lane;
     int ahead[4];
     auto request = [&](int j) {
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         const int pos = j * 128 + w * 32;
-        ahead[w] = (j >= from1 && pos + lane < c_mine) ? l_mine[pos] : j < from1 ? 0 : -1;      // (common steps are full)
+        ahead[w] = (pos + lane < c_mine) ? l_mine[pos] : -1;
       }
     };
     request(0);

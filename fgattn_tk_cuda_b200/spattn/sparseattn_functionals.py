@@ -69,8 +69,6 @@ def _sparse(out, query, key, value, mask, blocksz=128):
 
 def _sparse_bits(out, query, key, value, packed, n_valid):
     """One sparse step on a token mask of one bit per key, of which the first n_valid (None: all) count."""
-    if key.shape[2] >= 1 << 21:                            # more than the packed form counts
-        return _sparse(out, query, key, value, mask_utils._packedmask_to_lists(packed, n_valid))
     with mask_utils.nvtx_range("fgattn.sparse_attention"):
         spattn_interface.sp_attn_packed(out, query.contiguous(), key.contiguous(), value.contiguous(), packed.contiguous(),
                                         packed.shape[-1] * 8 if n_valid is None else n_valid)

@@ -144,9 +144,8 @@ int fgattn_sp_attn(void* o, const void* q, const void* k, const void* v, const i
 
 /* The same attention on a packed mask (one bit per key, see fgattn_pack_mask): query block i of a unit attends to the keys
  * whose bits are set in its row of row_bytes bytes, packed [B,H,ceil(seq/128),row_bytes]; bits from min(n_valid, kv_rows)
- * on do not count.  Keys that two neighbouring query blocks both keep are gathered once for the two.  `workspace`
- * (scratch) of fgattn_sp_attn_packed_workspace_bytes is needed.  kv_rows < 2^21.  Same result within rounding as fgattn_sp_attn on the
- * lists of fgattn_packedmask_to_lists. */
+ * on do not count.  `workspace` (scratch) of fgattn_sp_attn_packed_workspace_bytes is needed: the lists are written there.  Same
+ * result bit for bit as fgattn_sp_attn on the lists of fgattn_packedmask_to_lists. */
 size_t fgattn_sp_attn_packed_workspace_bytes(int batch, int heads, int seq, int kv_rows);
 int fgattn_sp_attn_packed(void* o, const void* q, const void* k, const void* v, const unsigned char* packed, int row_bytes,
                           int n_valid, int batch, int heads, int seq, int D, int kv_rows, float scale, void* workspace,

@@ -345,3 +345,40 @@ def test_items_of_the_last_wave_in_halves(D, S):
     _close(o2, parts(lambda *a: torch.ops.cuda_attn.sp_attn_packed(*a, n_kv), packed).cpu(), 8e-3, 5e-4)
     _close(o2, lists.cpu(), 8e-3, 5e-4)
     _capi().check()
+
+
+@pytest.mark.parametrize("H,S,D,n_kv", [(3, 256, 128, 1500), (2, 1000, 64, 4205), (5, 129, 128, 33), (2, 300, 64, 70001)])
+def test_packed_mask_gives_the_bits_of_its_lists(H, S, D, n_kv):
+    """sp_attn_packed takes a block's keys in ascending order, as the lists of the same bits have them: the same output bit
+    for bit (another order rounds other probabilities)."""
+    import fgattn_tk_cuda_b200.spattn  # noqa: F401  (registers torch.ops.cuda_attn)
+    from fgattn_tk_cuda_b200.spattn import mask_utils as mu
+    g = torch.Generator(device="cuda").manual_seed(S + n_kv)
+    q = torch.randn(1, H, S, D, generator=g, device="cuda").to(torch.bfloat16)
+    k, v = (torch.randn(1, H, n_kv, D, generator=g, device="cuda").to(torch.bfloat16) for _ in range(2))
+    width = 32 * ((n_kv + 31) // 32)
+    common = torch.rand(1, H, 1, width, generator=g, device="cuda") < 0.2
+    bits = common ^ (torch.rand(1, H, (S + 127) // 128, width, generator=g, device="cuda") < 0.1)
+    packed = mu.pack(bits)
+    o, lists = torch.full_like(q, float("nan")), torch.full_like(q, float("nan"))
+    torch.ops.cuda_attn.sp_attn_packed(o, q, k, v, packed, n_kv)
+    torch.ops.cuda_attn.sp_attn(lists, q, k, v, *mu.packedmask_to_indexmask_cuda(packed, n_kv))
+    _capi().check()
+    assert torch.equal(o, lists)
+
+
+@pytest.mark.parametrize("S,D", [(777, 64), (1408, 128)])
+def test_token_steps_give_the_bits_of_the_lists(S, D):
+    """The threshold step and the replay of kept bits: bit for bit sp_attn on the ascending lists of their masks."""
+    from fgattn_tk_cuda_b200 import synth
+    from fgattn_tk_cuda_b200.spattn import mask_utils as mu, sparseattn_functionals as sf
+    w = synth.Workload("t", 1, 3, S, D, "clustered", centroids=12, run=64, tau=0.5 / S, seed=S)
+    q, k, v = synth.make_qkv(w, device="cuda")
+    want = sf._sparse(sf._out(q), q, k, v, mu.qk_indexmask_cuda(q, k, w.tau))
+    assert torch.equal(sf.attn_computed_with_sparse_mask_cuda(q, k, v, thresh=w.tau, blocksz=128), want)
+    cache = mu.CompressedBitMaskCache([0])
+    sf.bitmaskcached_attn_cuda(q, k, v, 0, 0, mask_cache=cache, thresh=w.tau)
+    q2 = (q + 0.1 * torch.randn_like(q)).contiguous()
+    got = sf.bitmaskcached_attn_cuda(q2, k, v, 0, 1, mask_cache=cache, thresh=w.tau)
+    _capi().check()
+    assert torch.equal(got, sf._sparse(sf._out(q2), q2, k, v, cache.get_mask_from_cache(0)))
