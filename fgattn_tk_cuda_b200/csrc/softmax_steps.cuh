@@ -49,12 +49,15 @@ __device__ __forceinline__ void rescale_accumulator(uint32_t o_addr, float alpha
 //            L2 flushed between calls: 2 of 8 with P*V (C2 0.245 -> 0.232 ms, C4 5.33 -> 5.11 ms, C3 within
 //            2 %), 3 of 8 for the max / denominator pass (C3 2.49 -> 2.38 ms, C4 3.94 -> 3.45 ms); 4 of 8 is
 //            slower again: the polynomial costs ten issue slots per pair against two
+//   SKIP   : quarters of 32 columns that are negligible in all rows of a warp (kSkipLog2) take no exponentials.  The
+//            maximum passes over NaN, so a NaN score among negligible ones is skipped with them, and an infinite V row
+//            then meets a probability of zero instead of a tiny one.  Without: only quarters that the mask leaves out.
 //   quiet  : called before the accumulator is touched (waits for a product that may still be adding to it)
 //   loaded : called when the scores are in registers
 struct NoWait {
   __device__ __forceinline__ void operator()() const {}
 };
-template <int D, bool WRITE_P, int POLY = (WRITE_P ? 2 : 3), class Quiet = NoWait, class Loaded = NoWait>
+template <int D, bool WRITE_P, int POLY = (WRITE_P ? 2 : 3), bool SKIP = true, class Quiet = NoWait, class Loaded = NoWait>
 __device__ __forceinline__ void softmax_online_step(uint32_t s_addr, uint32_t p_addr, uint32_t o_addr, int valid0,
                                                     int valid1, float c, bool first, OnlineState& st, float& mx0,
                                                     float& mx1, const uint32_t* colmask = nullptr,
@@ -114,7 +117,8 @@ __device__ __forceinline__ void softmax_online_step(uint32_t s_addr, uint32_t p_
     // less than 2^-40 per entry relative to the running maximum -- under one fp32 ulp of the
     // denominator and of the output even summed over a whole row -- so its exponentials are
     // skipped and its probabilities are exact zeros.
-    const bool skip = __all_sync(0xffffffffu, fmaf(qmax[w], c, neg_m) < kSkipLog2);
+    const bool skip = SKIP ? __all_sync(0xffffffffu, fmaf(qmax[w], c, neg_m) < kSkipLog2)
+                           : colmask != nullptr && colmask[w] == 0u;
     if (skip) {
       if (WRITE_P) {
 #pragma unroll
@@ -166,10 +170,10 @@ __device__ __forceinline__ float quarter_max(const uint32_t (&r)[32]) {
 }
 
 // Probabilities of one 32-column quarter against the fixed offset -neg_m, packed to bf16 over r[0..15];
-// sum2 takes the even and the odd columns' sums.  POLY as in softmax_online_step.
-template <int POLY>
+// sum2 takes the even and the odd columns' sums.  POLY and SKIP as in softmax_online_step.
+template <int POLY, bool SKIP>
 __device__ __forceinline__ void quarter_probs(uint32_t (&r)[32], float qmax, float c, float neg_m, uint64_t& sum2) {
-  if (__all_sync(0xffffffffu, fmaf(qmax, c, neg_m) < kSkipLog2)) {
+  if (SKIP && __all_sync(0xffffffffu, fmaf(qmax, c, neg_m) < kSkipLog2)) {
 #pragma unroll
     for (int i = 0; i < 16; ++i) r[i] = 0u;
     return;
@@ -205,7 +209,7 @@ __device__ __forceinline__ void quarter_probs(uint32_t (&r)[32], float qmax, flo
 // pace a step.
 // `backwards` (warp-uniform): the quarters are taken last to first.  Only the first one taken is ever loaded again, so the
 // columns of the other half of the tile may be overwritten as soon as `loaded` has been called.
-template <int D, int POLY = 2, class Quiet = NoWait, class Loaded = NoWait>
+template <int D, int POLY = 2, bool SKIP = true, class Quiet = NoWait, class Loaded = NoWait>
 __device__ __forceinline__ void softmax_steady_step(uint32_t s_addr, uint32_t p_addr, uint32_t o_addr, float c,
                                                     OnlineState& st, float& mx0, float& mx1, Quiet quiet = Quiet(),
                                                     Loaded loaded = Loaded(), bool backwards = false) {
@@ -220,7 +224,7 @@ __device__ __forceinline__ void softmax_steady_step(uint32_t s_addr, uint32_t p_
 #pragma unroll
   for (int w = 1; w < 4; ++w) tmem_ld32(s_first + w * ds, r[w]);
   qm[0] = quarter_max(r[0]);
-  quarter_probs<POLY>(r[0], qm[0], c, neg_m, sum2);
+  quarter_probs<POLY, SKIP>(r[0], qm[0], c, neg_m, sum2);
 #pragma unroll
   for (int w = 1; w < 4; ++w) {
     tmem_ld_wait_for(r[w]);
@@ -235,7 +239,7 @@ __device__ __forceinline__ void softmax_steady_step(uint32_t s_addr, uint32_t p_
   auto finish = [&](float off, int from) {
 #pragma unroll
     for (int w = 0; w < 4; ++w) {
-      if (w >= from) quarter_probs<POLY>(r[w], qm[w], c, off, sum2);
+      if (w >= from) quarter_probs<POLY, SKIP>(r[w], qm[w], c, off, sum2);
       tmem_st16(p_first + w * dp, *reinterpret_cast<uint32_t(*)[16]>(&r[w][0]));
     }
     float sum0, sum1;

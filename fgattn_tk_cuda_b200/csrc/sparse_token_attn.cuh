@@ -307,10 +307,13 @@ sparse_token_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_co
       // full steps start their exponentials before the maximum is known (softmax_steps.cuh): top-k lists 0.720 -> 0.697 ms,
       // threshold lists 0.416 -> 0.399, D = 64 0.642 -> 0.629 and 0.351 -> 0.346, the same bits.  A share of the
       // exponentials on the FMA pipe: level to 5 % slower.
+      // Every listed key takes its exponential, however small: NaN and infinities of K and V rows reach the output.  Listed
+      // keys are hardly ever negligible for 32 rows, so the test for it cost more than it saved: threshold lists 0.390 ->
+      // 0.369 ms, D = 64 0.353 -> 0.337; top-k lists level and 0.642 -> 0.609.
       if (j > 0 && (live[0] & live[1] & live[2] & live[3]) == 0xffffffffu)
-        softmax_steady_step<D, 0>(s_addr, s_addr, o_addr, p.scale_log2, st, mx0, mx1);
+        softmax_steady_step<D, 0, false>(s_addr, s_addr, o_addr, p.scale_log2, st, mx0, mx1);
       else
-        softmax_online_step<D, true, 0>(s_addr, s_addr, o_addr, 64, 64, p.scale_log2, j == 0, st, mx0, mx1, live);
+        softmax_online_step<D, true, 0, false>(s_addr, s_addr, o_addr, 64, 64, p.scale_log2, j == 0, st, mx0, mx1, live);
       tc_fence_before();
       mbar_arrive(bar(TB_P_FULL + t));
       request(j + 1);

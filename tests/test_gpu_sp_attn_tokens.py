@@ -382,3 +382,42 @@ def test_token_steps_give_the_bits_of_the_lists(S, D):
     got = sf.bitmaskcached_attn_cuda(q2, k, v, 0, 1, mask_cache=cache, thresh=w.tau)
     _capi().check()
     assert torch.equal(got, sf._sparse(sf._out(q2), q2, k, v, cache.get_mask_from_cache(0)))
+
+
+@pytest.mark.parametrize("D", [64, 128])
+@pytest.mark.parametrize("pos", [40, 200, 290])
+def test_nan_and_infinity_of_negligible_keys_reach_the_output(D, pos):
+    """A listed key whose probability is tiny but not zero (2^-65 to 2^-92 of the row's largest) beside nothing but such keys:
+    NaN in its K row makes the output NaN, an infinity in its V row that column infinite, in the first step of a list
+    (entry 40), in a full one (200) and in a ragged last one (290 of 300)."""
+    import fgattn_tk_cuda_b200.spattn  # noqa: F401  (registers torch.ops.cuda_attn)
+    from fgattn_tk_cuda_b200.spattn import mask_utils as mu
+    H, S, n_kv, n = 2, 200, 640, 300
+    g = torch.Generator().manual_seed(pos)
+    q = torch.zeros(1, H, S, D)
+    k = torch.zeros(1, H, n_kv, D)
+    q[..., 0], k[..., 0] = 16.0, -16.0
+    v = torch.randn(1, H, n_kv, D, generator=g)
+    idx = torch.stack([torch.sort(torch.randperm(n_kv, generator=g)[:n]).values for _ in range(H * 2)])
+    idx = idx.to(torch.int32).view(1, H, 2, n)
+    for h in range(H):
+        k[0, h, idx[0, h, :, 5].long(), 0] = 16.0          # entry 5 of either block's list outweighs all others
+        k[0, h, idx[0, h, :, pos].long(), 0] = -16.0
+    cnt = torch.full((1, H, 2), n, dtype=torch.int32)
+    k_nan, v_inf = k.clone(), v.clone()
+    for h in range(H):
+        k_nan[0, h, idx[0, h, :, pos].long(), 1] = float("nan")
+        v_inf[0, h, idx[0, h, :, pos].long(), 3] = float("inf")
+    q, k, v, k_nan, v_inf = (x.to(torch.bfloat16).cuda() for x in (q, k, v, k_nan, v_inf))
+    idx, cnt = idx.cuda(), cnt.cuda()
+    bits = mu.indexmask_to_packedmask_cuda(idx, cnt, n_kv)
+    for attend in (lambda o, *a: torch.ops.cuda_attn.sp_attn(o, *a, idx, cnt),
+                   lambda o, *a: torch.ops.cuda_attn.sp_attn_packed(o, *a, bits, n_kv)):
+        o = torch.zeros_like(q)
+        attend(o, q, k_nan, v)
+        _capi().check()
+        assert torch.isnan(o).all()
+        attend(o, q, k, v_inf)
+        _capi().check()
+        assert torch.isinf(o[..., 3]).all()
+        assert torch.isfinite(torch.cat([o[..., :3], o[..., 4:]], -1)).all()
