@@ -12,14 +12,21 @@ from . import mask_utils
 spattn_interface = torch.ops.cuda_attn
 
 
-# Pairs of a query row and a key up to which the block-mask step is one operator: its kernels then take less time than two
-# operators, five allocations and their checks (4 heads of 1024 rows, D = 64: 38.3 -> 30.7 us).  The block maxima are at most
-# 1 / 16 of this in bytes (64 MiB).
-_ONE_CALL_PAIRS = 1 << 30
+# Pairs of a query row and a key, both in whole tiles (128 rows, 64 keys), up to which the block-mask step is one operator:
+# its kernels then take less time than two operators, five allocations and their checks.  Call after call, one operator
+# against two: 4 heads of 1024 rows (2^22 pairs) 26 / 52 us, 2 heads of 4096 (2^25) 65 / 65, 8 heads of 4096 level.  The
+# operator takes its block maxima at once, one float a row and 64 keys, which is 2 MiB here; above, the list build
+# works in chunks of heads that fit.
+_ONE_CALL_PAIRS = 1 << 25
 
 
 def _out(query):
     return torch.empty(query.shape, device=query.device, dtype=torch.bfloat16)
+
+
+def _one_call(query, key):
+    return query.is_cuda and query.dim() == 4 and key.dim() == 4 and query.shape[0] * query.shape[1] * \
+        (-(-query.shape[2] // 128) * 128) * (-(-key.shape[2] // 64) * 64) <= _ONE_CALL_PAIRS
 
 
 def _ml(query):
@@ -81,8 +88,7 @@ def attn_computed_with_sparse_mask_cuda(query, key, value, *args, **kwargs):
     if kwargs["blocksz"] == 128:
         packed = mask_utils._qk_packed_token_mask(query, key, kwargs["thresh"])
         return _sparse_bits(_out(query), query, key, value, packed, key.shape[2])
-    if kwargs["blocksz"] == 64 and query.is_cuda and query.dim() == 4 and key.dim() == 4 and \
-            query.shape[0] * query.shape[1] * query.shape[2] * key.shape[2] <= _ONE_CALL_PAIRS:
+    if kwargs["blocksz"] == 64 and _one_call(query, key):
         out = _out(query)
         spattn_interface.attn_block_mask(out, query.contiguous(), key.contiguous(), value.contiguous(), kwargs["thresh"])
         return out

@@ -321,3 +321,27 @@ def test_block_mask_step_in_one_operator(S, K, D):
     want = sf._sparse(sf._out(q), q, k, v, mu.qk_block_indexmask_cuda(q, k, w.tau))
     capi.check()
     assert torch.equal(o, want)
+
+
+@pytest.mark.parametrize("H,S,K,one_call", [(64, 1, 640, False), (200, 300, 1, False), (40, 130, 70, False), (2, 1024, 512, True)])
+def test_block_mask_step_counts_whole_tiles(monkeypatch, H, S, K, one_call):
+    """The one-operator step takes all its block maxima at once, for whole tiles of 128 rows and 64 keys: calls of few rows or few keys
+    and many heads, whose maxima are many times their pairs, go by the operators that work in chunks."""
+    from fgattn_tk_cuda_b200 import capi
+    from fgattn_tk_cuda_b200.spattn import mask_utils as mu, sparseattn_functionals as sf
+    monkeypatch.setattr(sf, "_ONE_CALL_PAIRS", 1 << 20)
+    assert (capi.block_scratch_bytes(1, H, S, K) <= (1 << 20) // 16) == one_call
+    g = torch.Generator(device="cuda").manual_seed(H)
+    q, k, v = (torch.randn(1, H, n, 64, generator=g, device="cuda").to(torch.bfloat16) for n in (S, K, K))
+    lists, calls = mu.qk_indexmask_cuda, []
+
+    def counted(*a, **kw):
+        calls.append(a)
+        return lists(*a, **kw)
+
+    monkeypatch.setattr(mu, "qk_indexmask_cuda", counted)
+    o = sf.attn_computed_with_sparse_mask_cuda(q, k, v, thresh=1e-3, blocksz=64)
+    assert bool(calls) != one_call
+    want = sf._sparse(sf._out(q), q, k, v, mu.qk_block_indexmask_cuda(q, k, 1e-3))
+    capi.check()
+    assert torch.equal(o, want)
