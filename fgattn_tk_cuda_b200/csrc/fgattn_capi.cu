@@ -1167,7 +1167,8 @@ int topk_select(int* kv_indices, int* kv_num_indices, int list_stride, uint32_t*
     return launch_behind(kern, dim3(unsigned(bh * nblk)), fg::kSelThreads, smem_sel, st, scores, s_stride, kv_seq_len, select_k,
                          k_pow2, cap, kv_indices, kv_num_indices, list_stride, bits, row_bytes / 4);
   };
-  return bits ? go(fg::topk_select_kernel<true>) : go(fg::topk_select_kernel<false>);
+  if (smem_sel > fg::kSelSmemOfThree) return bits ? go(fg::topk_select_kernel<true, 2>) : go(fg::topk_select_kernel<false, 2>);
+  return bits ? go(fg::topk_select_kernel<true, 3>) : go(fg::topk_select_kernel<false, 3>);
 }
 }  // namespace
 

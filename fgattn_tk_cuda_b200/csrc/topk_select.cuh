@@ -267,9 +267,13 @@ inline int select_capacity(int k) {
 // A sample of the row, 16 of every 128 bytes, gives a score that more than k and fewer than cap entries reach -- nearly
 // always; one sweep then collects those, and the count says whether it was so.  Rows where it was not go the general way
 // (below), which needs the range of the keys, one to three histogram sweeps and a sweep that collects.  3072 rows of
-// 32760 scores, k = 3276: 0.449 -> 0.235 ms with bits (the general way and the counting of places, all rows).
-template <bool BITS>
-__global__ void __launch_bounds__(kSelThreads, 3)
+// 32760 scores, k = 3276, means, scores and selection against the general way for all rows: 579 -> 402 us; with a NaN or one
+// score far above the others 880 -> 397; half of them equal 736 -> 572, all of few values 1195 -> 1240.
+// PER_SM: thread blocks that an SM's shared memory has room for.  Three leave 40 registers a thread, a few too few for the
+// general way: 8192 keys of rows of equal scores, where two fit anyway, 1.67 -> 1.58 ms with the registers of two.
+constexpr int kSelSmemOfThree = 66 * 1024;
+template <bool BITS, int PER_SM>
+__global__ void __launch_bounds__(kSelThreads, PER_SM)
 topk_select_kernel(const float* scores, int s_stride, int n, int k, int k_pow2, int cap, int* idx,
                    int* cnt, int list_stride, uint32_t* bits, int row_words) {
   // (key << 32 | ~index), cap entries and room for a bin's; then cap slots, or the row's bits
@@ -368,9 +372,12 @@ topk_select_kernel(const float* scores, int s_stride, int n, int k, int k_pow2, 
     to_bin = float(kSelBins - 1) / (f_hi - float_of_order_key(key_lo));
     return to_bin > 0.f && to_bin < 1e30f;
   };
-  auto bin_of_key = [&](uint32_t key) -> int { return max(0, min(kSelBins - 1, int((f_hi - float_of_order_key(key)) * to_bin))); };
+  // (scores above f_hi and NaN go to the first bin)
+  auto bin_of_key = [&](uint32_t key) -> int {
+    return int(fminf(fmaxf((f_hi - float_of_order_key(key)) * to_bin, 0.f), float(kSelBins - 1)));
+  };
 
-  // The k largest of the m >= k entries in sel, whose keys lie in [key_lo, key_hi], by counting: the entries are counted into
+  // The k largest of the m >= k entries in sel, whose keys are key_lo or more and most of them key_hi or less, by counting: the entries are counted into
   // 2048 bins of equal width over their range of scores (a monotone map, so a larger bin holds smaller scores), every
   // entry gets a slot in its bin, and inside a bin -- a few entries -- an entry's place is the number of larger ones.
   // Five barriers where a bitonic sort of 4096 entries takes 78 passes: 3276 of 32760 keys for 3072 rows, the whole
@@ -430,17 +437,20 @@ topk_select_kernel(const float* scores, int s_stride, int n, int k, int k_pow2, 
     return true;
   };
 
+  int sort_n = 0;                                        // entries of sel to sort, a power of two (zeros fill up); none yet
   // ---- the short way
   {
-    const int m4 = (n4 + 7) >> 3;                          // float4s of the sample
+    // The sample: of every 32 entries the four at a place that changes from one to the next, so that keys which differ by
+    // their place in the rows of an image, of a multiple of 32 keys, are like their sample.  A fixed place: 3072 rows of
+    // 32760 scores, k = 3276, where 4 of every 32 keys stand out 648 us for the whole selection instead of 428.
+    const int m4 = n >> 5;                                 // float4s of the sample
     uint32_t kmin = 0xffffffffu, kmax = 0u;
     auto sample = [&](auto&& f) {
       for (int i = tid; i < m4; i += kSelThreads) {
-        const float4 v = row4[8 * i];
+        const float4 v = row4[8 * i + ((uint32_t(i) * 0x9E3779B1u) >> 29)];
         const float x[4] = {v.x, v.y, v.z, v.w};
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (32 * i + e < n) f(float_order_key(x[e]));
+        for (int e = 0; e < 4; ++e) f(float_order_key(x[e]));
       }
     };
     sample([&](uint32_t key) {
@@ -449,26 +459,26 @@ topk_select_kernel(const float* scores, int s_stride, int n, int k, int k_pow2, 
     });
     key_range(kmin, kmax);
     const uint32_t lo_key = s_lo, hi_key = s_hi;
-    const int m = 4 * (m4 - 1) + min(4, n - 32 * (m4 - 1));
+    const int m = 4 * m4;
     // the sample's rank of a score that (k + cap) / 2 entries of the row reach
     const int rank = int((long long)(k + cap) * m / (2 * n));
     if (rank >= 1 && rank < m && set_bins(hi_key, lo_key)) {
       clear_hist();
-      if (tid == 0) { s_count = 0; s_max = 0u; s_rem = kSelBins; }
+      if (tid == 0) { s_count = 0; s_rem = kSelBins; }
       __syncthreads();
       sample([&](uint32_t key) { atomicAdd(&hist[bin_of_key(key)], 1); });
       __syncthreads();
       scan_hist();
-      // the first bin that starts at or past that rank: its upper edge is the threshold
+      // the first bin that starts at or past that rank: its upper edge is the threshold, unless equal scores make it
+      // reach more entries than there is room for
 #pragma unroll
       for (int u = 0; u < 4; ++u) {
         const int b = 4 * tid + u;
-        if (b > 0 && hist[b] >= rank && hist[b - 1] < rank) s_rem = b;
+        if (b > 0 && hist[b] >= rank && hist[b - 1] < rank && (long long)hist[b] * n <= (long long)cap * m) s_rem = b;
       }
       __syncthreads();
       if (s_rem < kSelBins) {
         const uint32_t from = float_order_key(f_hi - float(s_rem) / to_bin);
-        uint32_t top = 0u;
         // reach(x): the score counts.  A threshold above zero is compared as the integer that its bits are (the larger of two
         // positive floats, NaN included, is the larger integer, and negative ones are negative integers): one instruction
         // an entry where the order-preserving image takes four.
@@ -511,10 +521,8 @@ topk_select_kernel(const float* scores, int s_stride, int n, int k, int k_pow2, 
 #pragma unroll
               for (int e = 0; e < 4; ++e) {
                 if ((take >> (4 * u + e)) & 1u) {
-                  const uint32_t key = float_order_key(x[e]);
-                  top = max(top, key);
                   if (at < cap)
-                    sel[at] = (static_cast<unsigned long long>(key) << 32) |
+                    sel[at] = (static_cast<unsigned long long>(float_order_key(x[e])) << 32) |
                               uint32_t(~uint32_t(4 * (base + u * kSelThreads + tid) + e));
                   ++at;
                 }
@@ -528,13 +536,19 @@ topk_select_kernel(const float* scores, int s_stride, int n, int k, int k_pow2, 
         } else {
           collect([&](float x) { return float_order_key(x) >= from; });
         }
-        top = __reduce_max_sync(0xffffffffu, top);
-        if (lane == 0) atomicMax(&s_max, top);
         __syncthreads();
         const int got = s_count;
-        const uint32_t max_key = s_max;
         __syncthreads();
-        if (got >= k && got <= cap && finish_by_counting(got, max_key, from)) return;
+        if (got >= k && got <= cap) {
+          // counted up to the sample's largest score: the few above it, NaN among them, share a bin
+          if (finish_by_counting(got, hi_key, from)) return;
+          int size = 2;
+          while (size < got) size <<= 1;
+          if (size <= cap) {
+            for (int i = got + tid; i < size; i += kSelThreads) sel[i] = 0ull;
+            sort_n = size;
+          }
+        }
       }
     }
     __syncthreads();
@@ -547,117 +561,120 @@ topk_select_kernel(const float* scores, int s_stride, int n, int k, int k_pow2, 
   // of a row into two or three bins of its leading byte and serialise the shared-memory counters), picks the bin that
   // holds the k-th largest and narrows the interval to it, until the bin and everything above it fit the sort buffer
   // (usually after one histogram sweep) or the bins are one key wide.
-  // ---- key range of the row
-  uint32_t kmin = 0xffffffffu, kmax = 0u;
-  sweep([&](uint32_t key, int, bool live) {
-    if (live) {
-      kmin = min(kmin, key);
-      kmax = max(kmax, key);
-    }
-  });
-  key_range(kmin, kmax);
-  if (tid == 0) {
-    s_max = s_hi;
-    s_rem = k;
-  }
-  __syncthreads();
-
-  // ---- narrow [lo, hi] around the k-th largest key.  hi - lo < 2^shift after a sweep, so shift goes from 21 at most to
-  // 10 to 0: three sweeps at most.
-  while (true) {
-    const uint32_t lo = s_lo, hi = s_hi;
-    const int rem = s_rem;
-    const uint32_t width = hi - lo;                                    // keys in the interval - 1
-    const int shift = max(0, (32 - __clz(width | 1u)) - 11);           // (hi - lo) >> shift < 2048
-    for (int i = tid; i < kSelBins; i += kSelThreads) hist[i] = 0;
-    __syncthreads();
+  if (sort_n == 0) {
+    // ---- key range of the row
+    uint32_t kmin = 0xffffffffu, kmax = 0u;
     sweep([&](uint32_t key, int, bool live) {
-      if (live && key >= lo && key <= hi) atomicAdd(&hist[(key - lo) >> shift], 1);
+      if (live) {
+        kmin = min(kmin, key);
+        kmax = max(kmax, key);
+      }
     });
+    key_range(kmin, kmax);
+    if (tid == 0) {
+      s_max = s_hi;
+      s_rem = k;
+    }
     __syncthreads();
-    if (warp == 0) {
-      // lane L owns the 64 bins [2048 - 64 (L + 1), 2048 - 64 L): lane 0 holds the largest keys
-      constexpr int kPer = kSelBins / 32;
-      const int b0 = kSelBins - kPer * (lane + 1);
-      int mine = 0;
-      for (int b = 0; b < kPer; ++b) mine += hist[b0 + b];
-      int incl = mine;
+
+    // ---- narrow [lo, hi] around the k-th largest key.  hi - lo < 2^shift after a sweep, so shift goes from 21 at most to
+    // 10 to 0: three sweeps at most.
+    while (true) {
+      const uint32_t lo = s_lo, hi = s_hi;
+      const int rem = s_rem;
+      const uint32_t width = hi - lo;                                    // keys in the interval - 1
+      const int shift = max(0, (32 - __clz(width | 1u)) - 11);           // (hi - lo) >> shift < 2048
+      for (int i = tid; i < kSelBins; i += kSelThreads) hist[i] = 0;
+      __syncthreads();
+      sweep([&](uint32_t key, int, bool live) {
+        if (live && key >= lo && key <= hi) atomicAdd(&hist[(key - lo) >> shift], 1);
+      });
+      __syncthreads();
+      if (warp == 0) {
+        // lane L owns the 64 bins [2048 - 64 (L + 1), 2048 - 64 L): lane 0 holds the largest keys
+        constexpr int kPer = kSelBins / 32;
+        const int b0 = kSelBins - kPer * (lane + 1);
+        int mine = 0;
+        for (int b = 0; b < kPer; ++b) mine += hist[b0 + b];
+        int incl = mine;
 #pragma unroll
-      for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
-      }
-      const bool here = incl >= rem && incl - mine < rem;              // exactly one lane
-      if (here) {
-        int r = rem - (incl - mine), b = kPer - 1;
-        for (; b > 0; --b) {
-          if (hist[b0 + b] >= r) break;
-          r -= hist[b0 + b];
+        for (int o = 1; o < 32; o <<= 1) {
+          const int t = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += t;
         }
-        const uint32_t nlo = lo + (uint32_t(b0 + b) << shift);
-        s_lo = nlo;
-        s_hi = nlo + min(hi - nlo, (1u << shift) - 1u);          // (the keys of NaNs reach 2^32 - 1: no wrap)
-        s_rem = r;
-        s_ties = hist[b0 + b];
+        const bool here = incl >= rem && incl - mine < rem;              // exactly one lane
+        if (here) {
+          int r = rem - (incl - mine), b = kPer - 1;
+          for (; b > 0; --b) {
+            if (hist[b0 + b] >= r) break;
+            r -= hist[b0 + b];
+          }
+          const uint32_t nlo = lo + (uint32_t(b0 + b) << shift);
+          s_lo = nlo;
+          s_hi = nlo + min(hi - nlo, (1u << shift) - 1u);          // (the keys of NaNs reach 2^32 - 1: no wrap)
+          s_rem = r;
+          s_ties = hist[b0 + b];
+        }
+      }
+      __syncthreads();
+      // stop as soon as everything from the chosen bin upwards fits the sort buffer: the sort then
+      // orders the bin's entries too and the first k sorted entries are the answer
+      if (shift == 0 || (k - s_rem) + s_ties <= k_pow2) break;
+    }
+    const uint32_t kth = s_lo;                             // lowest key taken; s_rem of the s_ties entries in
+                                                           // [kth, s_hi] are needed (s_hi == kth after a full narrowing)
+    const int rem = s_rem, n_gt = k - rem;
+    __syncthreads();
+
+    if (tid == 0) { s_count = 0; s_base = 0; }
+    for (int i = tid; i < k_pow2; i += kSelThreads) sel[i] = 0ull;
+    __syncthreads();
+    if (n_gt + s_ties <= k_pow2) {
+      // ---- common case: everything >= kth fits the sort buffer; the sort puts ties in index order.
+      // One shared-counter update per warp and sweep slot.
+      sweep([&](uint32_t key, int i, bool live) {
+        const bool take = live && key >= kth;
+        const uint32_t bal = __ballot_sync(0xffffffffu, take);
+        if (bal) {
+          int base = 0;
+          if (lane == __ffs(bal) - 1) base = atomicAdd(&s_count, __popc(bal));
+          base = __shfl_sync(0xffffffffu, base, __ffs(bal) - 1);
+          if (take)
+            sel[base + __popc(bal & ((1u << lane) - 1u))] =
+                (static_cast<unsigned long long>(key) << 32) | uint32_t(~uint32_t(i));
+        }
+      });
+    } else {
+      // ---- many ties at the k-th key: entries above it in any order, then the first `rem` ties by index
+      for (int i0 = 0; i0 < n; i0 += kSelThreads) {
+        const int i = i0 + tid;
+        const uint32_t key = (i < n) ? float_order_key(row[i]) : 0u;
+        if (i < n && key > kth) {
+          const int pos = atomicAdd(&s_count, 1);
+          sel[pos] = (static_cast<unsigned long long>(key) << 32) | uint32_t(~uint32_t(i));
+        }
+        const int tie = (i < n && key == kth) ? 1 : 0;
+        const uint32_t bal = __ballot_sync(0xffffffffu, tie);
+        if (lane == 0) warp_tot[warp] = __popc(bal);
+        __syncthreads();
+        int off = s_base;
+        for (int w = 0; w < warp; ++w) off += warp_tot[w];
+        off += __popc(bal & ((1u << lane) - 1u));
+        if (tie && off < rem)
+          sel[n_gt + off] = (static_cast<unsigned long long>(key) << 32) | uint32_t(~uint32_t(i));
+        __syncthreads();
+        if (tid == kSelThreads - 1) s_base = off + tie;
+        __syncthreads();
       }
     }
     __syncthreads();
-    // stop as soon as everything from the chosen bin upwards fits the sort buffer: the sort then
-    // orders the bin's entries too and the first k sorted entries are the answer
-    if (shift == 0 || (k - s_rem) + s_ties <= k_pow2) break;
-  }
-  const uint32_t kth = s_lo;                             // lowest key taken; s_rem of the s_ties entries in
-                                                         // [kth, s_hi] are needed (s_hi == kth after a full narrowing)
-  const int rem = s_rem, n_gt = k - rem;
-  __syncthreads();
 
-  if (tid == 0) { s_count = 0; s_base = 0; }
-  for (int i = tid; i < k_pow2; i += kSelThreads) sel[i] = 0ull;
-  __syncthreads();
-  if (n_gt + s_ties <= k_pow2) {
-    // ---- common case: everything >= kth fits the sort buffer; the sort puts ties in index order.
-    // One shared-counter update per warp and sweep slot.
-    sweep([&](uint32_t key, int i, bool live) {
-      const bool take = live && key >= kth;
-      const uint32_t bal = __ballot_sync(0xffffffffu, take);
-      if (bal) {
-        int base = 0;
-        if (lane == __ffs(bal) - 1) base = atomicAdd(&s_count, __popc(bal));
-        base = __shfl_sync(0xffffffffu, base, __ffs(bal) - 1);
-        if (take)
-          sel[base + __popc(bal & ((1u << lane) - 1u))] =
-              (static_cast<unsigned long long>(key) << 32) | uint32_t(~uint32_t(i));
-      }
-    });
-  } else {
-    // ---- many ties at the k-th key: entries above it in any order, then the first `rem` ties by index
-    for (int i0 = 0; i0 < n; i0 += kSelThreads) {
-      const int i = i0 + tid;
-      const uint32_t key = (i < n) ? float_order_key(row[i]) : 0u;
-      if (i < n && key > kth) {
-        const int pos = atomicAdd(&s_count, 1);
-        sel[pos] = (static_cast<unsigned long long>(key) << 32) | uint32_t(~uint32_t(i));
-      }
-      const int tie = (i < n && key == kth) ? 1 : 0;
-      const uint32_t bal = __ballot_sync(0xffffffffu, tie);
-      if (lane == 0) warp_tot[warp] = __popc(bal);
-      __syncthreads();
-      int off = s_base;
-      for (int w = 0; w < warp; ++w) off += warp_tot[w];
-      off += __popc(bal & ((1u << lane) - 1u));
-      if (tie && off < rem)
-        sel[n_gt + off] = (static_cast<unsigned long long>(key) << 32) | uint32_t(~uint32_t(i));
-      __syncthreads();
-      if (tid == kSelThreads - 1) s_base = off + tie;
-      __syncthreads();
-    }
+    const int m = (n_gt + s_ties <= k_pow2) ? n_gt + s_ties : k;
+    const uint32_t key_top = s_max;
+    if (finish_by_counting(m, key_top, kth)) return;
+    __syncthreads();
+    sort_n = k_pow2;
   }
-  __syncthreads();
-
-  const int m = (n_gt + s_ties <= k_pow2) ? n_gt + s_ties : k;
-  const uint32_t key_top = s_max;
-  if (finish_by_counting(m, key_top, kth)) return;
-  __syncthreads();
 
   // ---- bitonic sort, descending: the first k entries are the answer.  The passes of strides up to 32 stay inside groups
   // of 64 entries: a warp takes a group through all of them in registers, two entries a lane, and only the passes
@@ -666,10 +683,10 @@ topk_select_kernel(const float* scores, int s_stride, int n, int k, int k_pow2, 
   // alone: half of the scores equal, 3276 keys 1.234 -> 1.251 ms, now 1.156; 8192 keys 1.906 -> 2.102, now 1.826; one
   // score at 30 deviations 1.017 -> 1.027, now 0.849, and 1.893 -> 1.990, now 1.550.
   auto in_group = [&](int size_from, int size_to) {        // the passes of these sizes whose strides are 32 or less
-    for (int g = warp * 64; g < k_pow2; g += (kSelThreads / 32) * 64) {
+    for (int g = warp * 64; g < sort_n; g += (kSelThreads / 32) * 64) {
       unsigned long long x[2];
 #pragma unroll
-      for (int h = 0; h < 2; ++h) x[h] = (g + 32 * h + lane < k_pow2) ? sel[g + 32 * h + lane] : 0ull;
+      for (int h = 0; h < 2; ++h) x[h] = (g + 32 * h + lane < sort_n) ? sel[g + 32 * h + lane] : 0ull;
       for (int size = size_from; size <= size_to; size <<= 1) {
         if (size >= 64) {
           const bool desc = (g & size) == 0;
@@ -688,14 +705,14 @@ topk_select_kernel(const float* scores, int s_stride, int n, int k, int k_pow2, 
       }
 #pragma unroll
       for (int h = 0; h < 2; ++h)
-        if (g + 32 * h + lane < k_pow2) sel[g + 32 * h + lane] = x[h];
+        if (g + 32 * h + lane < sort_n) sel[g + 32 * h + lane] = x[h];
     }
     __syncthreads();
   };
   in_group(2, 64);                                         // (entries past the end of a short list count as zeros, the smallest)
-  for (int size = 128; size <= k_pow2; size <<= 1) {
+  for (int size = 128; size <= sort_n; size <<= 1) {
     for (int stride = size >> 1; stride > 32; stride >>= 1) {
-      for (int t = tid; t < (k_pow2 >> 1); t += kSelThreads) {
+      for (int t = tid; t < (sort_n >> 1); t += kSelThreads) {
         const int lo = 2 * t - (t & (stride - 1)), hi = lo + stride;
         const bool desc = (lo & size) == 0;
         const unsigned long long a = sel[lo], b = sel[hi];

@@ -297,3 +297,28 @@ def test_topk_attention_takes_keys_by_score(S, D, select_k):
     _capi().check()
     assert torch.equal(o, want)
     assert not torch.equal(by_key, want)
+
+
+@pytest.mark.parametrize("kind", ["above", "below", "outliers", "outlier_in_sample", "infinite", "piled"])
+@pytest.mark.parametrize("S,select_k", [(31, 7), (32, 5), (100, 20), (4097, 100), (20001, 2000), (20000, 3300), (33000, 8192)])
+def test_topk_of_rows_unlike_their_sample(kind, S, select_k):
+    """Scores whose sample (four of every 32, at a place that changes) lies above or below the rest, or holds all or none
+    of a few scores far above the others, and scores that pile up just under the largest: every way from the sample to the list."""
+    g = torch.Generator().manual_seed(S + select_k)
+    x = torch.randn(S, generator=g).to(torch.bfloat16).float()
+    i = torch.arange(S)
+    sampled = (i // 4 % 8 == (i // 32 * 0x9E3779B1 % (1 << 32)) >> 29) & (i < S // 32 * 32)
+    if kind == "above":
+        x[sampled] += 16
+    elif kind == "below":
+        x[sampled] -= 16
+    elif kind in ("outliers", "infinite"):
+        x[torch.nonzero(~sampled).flatten()[:: max(1, S // 20)][:20]] = 2.0 ** (60 if kind == "outliers" else 127)
+    elif kind == "outlier_in_sample":
+        x[torch.nonzero(sampled).flatten()[:1]] = 2.0 ** 60
+    else:
+        x[torch.rand(S, generator=g) < 0.9 * select_k / S] = 2.5
+        x[torch.nonzero(sampled).flatten()[:3]] = 64.0
+    x = x.to(torch.bfloat16).float()
+    got = _list_of_scores(torch.stack([x, torch.zeros_like(x)], 1), 0.0, select_k, q0=4.0)
+    assert torch.equal(got, torch.sort(4.0 * x, descending=True, stable=True).indices[:select_k])
