@@ -180,9 +180,12 @@ int launch_dense_k(const CUtensorMap& mq, const CUtensorMap& mk, const CUtensorM
 }
 
 constexpr int kPersistMaxKeyTiles = 8;     // persistent CTAs up to 1024 keys
-// Persistent CTAs at D = 64: the scores rotate above 256 keys.  One buffer a tile against rotating scores: 16384 rows of
-// 24 heads, 77 keys level, 256 keys 55.4 / 56.4 us; 32768 rows of 40 heads, 512 keys 275 / 262 us
-constexpr int kOneBufferMaxKeyTiles = 2;
+// Persistent CTAs at D = 64: the scores rotate above 512 keys.  One buffer a tile against rotating scores, 16384 rows of
+// 24 heads, q and k of deviation 1 / 2 / 3: 300 keys 79 / 79 / 81 against 79 / 87 / 86 us, 512 keys 97 / 99 / 103 against 93 / 106 /
+// 112 and on clustered keys 46.0 against 48.1 (4096 rows), 640 keys 115 / 128 / 136 against 112 / 125 / 132.  In items of three or
+// four key tiles the offset of the exponentials moves in most steps unless scores lie close together, and a rotating step
+// then takes its first quarter twice and waits for the product before.
+constexpr int kOneBufferMaxKeyTiles = 4;
 // The max / denominator pass alone stays persistent up to 2048 keys: measured against its one-item kernel
 // (maxq_pass.cuh) at 32768 queries x 40 heads, D = 128 / 64: 1280 keys 16 / 12 % faster, 1536 keys 13 / 6 %,
 // 2048 keys 10 / 4 %, 3072 keys level / 1 % slower
