@@ -159,3 +159,62 @@ def test_replaced_reading_of_a_kept_mask_is_called(monkeypatch):
     monkeypatch.setattr(mask_utils.CompressedBitMaskCache, "get_mask_from_cache", own)
     _replay(_bit_cache(SKV))
     assert calls == [0, 0, 0]
+
+
+def _added(name, **change):
+    a = dict(good(), packed=t(B, H, NQB128, 28, dtype=torch.uint8), n_valid=SKV, select=100, blocksz=128, tau=1e-3)
+    a.update(change)
+    if name == "sp_attn_packed":
+        return ops.sp_attn_packed(a["o"], a["q"], a["k"], a["v"], a["packed"], a["n_valid"])
+    if name == "topk_packed":
+        return ops.topk_packed(a["packed"], a["q"], a["k"], a["select"], a["blocksz"])
+    return ops.attn_block_mask(a["o"], a["q"], a["k"], a["v"], a["tau"])
+
+
+_QKV_BAD = [dict(k=t(B, H + 1, SKV, D)), dict(k=t(B, H, SKV, 128)), dict(q=t(B, H, S, 96)), dict(k=t(B, H, 0, D)),
+            dict(q=t(B, H, S, D, dtype=torch.float16))]
+_VO_BAD = [dict(v=t(B, H, SKV - 8, D)), dict(o=t(B, H, S - 1, D)), dict(o=t(B, H, S, D, dtype=torch.float32))]
+_PACKED_BAD = [dict(packed=t(B, H, NQB128 + 1, 28, dtype=torch.uint8)), dict(packed=t(B, H, NQB128, 28, dtype=torch.int32)),
+               dict(packed=t(B * H, NQB128, 28, dtype=torch.uint8)), dict(packed=t(B, H, NQB128, 56, dtype=torch.uint8)[..., ::2])]
+
+
+@pytest.mark.parametrize("name,bad", [("attn_block_mask", _QKV_BAD + _VO_BAD + [dict(tau=0.0), dict(tau=-1.0)]),
+                                      ("sp_attn_packed", _QKV_BAD + _VO_BAD + _PACKED_BAD + [dict(n_valid=-1)]),
+                                      ("topk_packed", _QKV_BAD + _PACKED_BAD + [
+                                          dict(packed=t(B, H, NQB128, 24, dtype=torch.uint8)),        # fewer bits than keys
+                                          dict(packed=t(B, H, NQB128, 26, dtype=torch.uint8)),        # not whole words
+                                          dict(select=0), dict(select=SKV + 1), dict(blocksz=0), dict(blocksz=64)])])
+def test_operators_on_bits_and_in_one_call_refuse_wrong_arguments(name, bad):
+    assert _added(name) is None
+    for change in bad:
+        with pytest.raises(RuntimeError):
+            _added(name, **change)
+
+
+def test_replaced_lists_of_a_kept_mask_are_read(monkeypatch):
+    """A step goes by the kept bits only as long as nothing that hands out their lists has been replaced."""
+    from fgattn_tk_cuda_b200.spattn import mask_utils
+    calls = []
+
+    def own(*layer):
+        calls.append(layer[-1])
+        return good()["ti"], good()["tc"]
+
+    plain = _bit_cache(SKV)
+    assert plain.reads_bits()
+    on_object, reader = _bit_cache(SKV), _bit_cache(SKV)
+    on_object.get_lists = own
+    reader.list_reader = lambda: own
+
+    class Sub(mask_utils.CompressedBitMaskCache):
+        get_lists = own
+
+    sub = Sub([0])
+    sub.cache = plain.cache
+    for cache in (on_object, reader, sub):
+        assert not cache.reads_bits()
+        _replay(cache)
+    monkeypatch.setattr(mask_utils.CompressedBitMaskCache, "get_lists", own)
+    assert not plain.reads_bits()
+    _replay(plain)
+    assert calls == [0, 0, 0, 0]
