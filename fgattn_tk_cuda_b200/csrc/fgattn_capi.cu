@@ -1163,7 +1163,8 @@ int topk_select(int* kv_indices, int* kv_num_indices, int list_stride, uint32_t*
   while (k_pow2 < select_k) k_pow2 <<= 1;
   const int cap = fg::select_capacity(select_k);
   const int smem_sel = 8 * (cap + int(fg::kSelBinSort)) + (bits ? row_bytes : 2 * cap);
-  if (smem_sel > 200 * 1024) return FGATTN_UNSUPPORTED;    // rows of more than 800000 bits beside the largest selection
+  // the row's bits are put together beside the selected entries: with 8192 of those rows of 122368 bytes at most
+  if (smem_sel > 200 * 1024) return FGATTN_UNSUPPORTED;
   auto go = [&](auto kern) -> int {
     int rr = set_smem(kern, smem_sel);
     if (rr) return rr;

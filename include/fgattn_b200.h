@@ -305,7 +305,10 @@ int fgattn_topk_indices(int* kv_indices, int* kv_num_indices, int list_stride, c
                         float scale, void* scratch, size_t scratch_bytes, void* stream);
 
 /* The same selection as a packed mask (one bit per key, rows of row_bytes bytes, a multiple of 4 and at least
- * kv_seq_len / 8), for a program that asks for the set of keys and not for their order.  packed [B,H,ceil(seq/blocksz),row_bytes], 4-byte aligned. */
+ * kv_seq_len / 8), for a program that asks for the set of keys and not for their order.  packed [B,H,ceil(seq/blocksz),row_bytes],
+ * 4-byte aligned.  A row is put together in shared memory beside the selected entries: FGATTN_UNSUPPORTED where
+ * 8 * (cap + 64) + row_bytes exceeds 200 KiB, cap = max(1024, the power of two from select_k on, 1.25 * select_k rounded up to
+ * a multiple of 64), so rows of up to 122368 bytes (978944 keys) are taken at every select_k. */
 int fgattn_topk_packed(unsigned char* packed, int row_bytes, const void* q, const void* k, int select_k, int batch, int heads,
                        int seq, int D, int blocksz, int kv_rows, int kv_seq_len, float scale, void* scratch,
                        size_t scratch_bytes, void* stream);

@@ -322,3 +322,20 @@ def test_topk_of_rows_unlike_their_sample(kind, S, select_k):
     x = x.to(torch.bfloat16).float()
     got = _list_of_scores(torch.stack([x, torch.zeros_like(x)], 1), 0.0, select_k, q0=4.0)
     assert torch.equal(got, torch.sort(4.0 * x, descending=True, stable=True).indices[:select_k])
+
+
+def test_topk_as_bits_refuses_rows_beside_which_the_selection_has_no_room():
+    """A row's bits are put together in shared memory beside the selected entries: 8 * (1.25 k + 64) + row bytes <= 200 KiB."""
+    import fgattn_tk_cuda_b200.spattn  # noqa: F401  (registers torch.ops.cuda_attn)
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q = torch.randn(1, 1, 128, 64, generator=g, device="cuda").to(torch.bfloat16)
+    k = torch.randn(1, 1, 9000, 64, generator=g, device="cuda").to(torch.bfloat16)
+    room = 200 * 1024 - 8 * (10240 + 64)
+    with pytest.raises(RuntimeError, match="topk_packed failed"):
+        torch.ops.cuda_attn.topk_packed(torch.zeros(1, 1, 1, room + 4, dtype=torch.uint8, device="cuda"), q, k, 8192, 128)
+    packed = torch.full((1, 1, 1, room), 0xA5, dtype=torch.uint8, device="cuda")
+    torch.ops.cuda_attn.topk_packed(packed, q, k, 8192, 128)
+    _capi().check()
+    bits = torch.zeros(1, 8 * room, dtype=torch.uint8, device="cuda")
+    _capi().unpack_mask(bits, packed.view(1, room))
+    assert int(bits.sum()) == 8192 and int(bits[:, 9000:].sum()) == 0
