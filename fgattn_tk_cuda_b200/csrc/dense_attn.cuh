@@ -79,9 +79,9 @@ enum : int {
   BAR_V_EMPTY = 13,  // +stage
   BAR_S_FULL = 17,   // +tile*2+buf
   BAR_S_EMPTY = 21,  // +tile*2+buf (with rotating scores +tile*2+step parity: the step's scores are in registers)
-  BAR_P_FULL = 25,   // +tile*2 (+step parity with rotating score buffers)
+  BAR_P_FULL = 25,   // +tile*2 (+step parity with rotating scores)
   BAR_O_FULL = 29,   // +tile
-  BAR_PV_DONE = 31,  // +tile: rotating score buffers only, the tile's last P V product has been executed
+  BAR_PV_DONE = 31,  // +tile: rotating scores only, the tile's last P V product has been executed
   BAR_Q_EMPTY = 33,  // the item's last Q K^T product has been executed
   BAR_COUNT = 34
 };
@@ -103,9 +103,10 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
   // before ends, and what is left in the chain is the softmax itself.  Against three
   // 128-column buffers that both tiles went round, where a softmax warp waited 886 of 2680 clocks a step for its scores:
   // (2, 16, 4096, 64) 212 -> 199 us, 24 heads of 8192 rows 598 -> 564, clustered keys at (4, 24, 12345, 64) 4.88 -> 4.52 ms;
-  // where the offset moves in most tiles (q and k of deviation 3) 238 -> 241 us.
+  // q and k of deviation 2 / 3 / 6, where the offset moves in some to most tiles: 232 / 247 / 255 -> 238 / 249 / 255 us.  (Taking
+  // softmax_online_step wherever the step before has moved the offset: twice the time where the two mix, 460 us.)
   // The persistent form rotates where an item is long enough (kOneBufferMaxKeyTiles of the launcher).
-  static_assert(!ROT || (HAS_V && D == 64), "room for a third score buffer");
+  static_assert(!ROT || (HAS_V && D == 64), "192 columns a query tile for scores and probabilities");
   constexpr uint32_t kColO = ROT ? 384 : 256, kOStride = ROT ? 64 : 128;
   constexpr bool TWO_ISS = (HAS_V && D == 128) || MODE == kML;   // one UMMA issuer warp per query tile ...
   constexpr int kTwoIssMinTiles = 64;                            // ... from 8192 keys on: with fewer the second
@@ -270,8 +271,8 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
     // scores), and an issuer that serves both tiles in turn reaches a tile's probabilities late whenever it is
     // busy with the other tile's waits and commits (C3 3.38 -> 3.20 ms).  The max / denominator mode gains the
     // same way (a freed score buffer is refilled at once: C3 2.32 -> 2.18 ms, C4 3.43 -> 3.36 ms).  With V at
-    // D = 64 one warp serves both tiles, whose units share the rotating buffers in one order (with one buffer a tile
-    // two issuers were 1 % slower), as in the token-mask mode and for key sequences under 8192.  (The gain depends on
+    // D = 64 one warp serves both tiles, whose products it issues in turn (with one score buffer a tile two issuers
+    // were 1 % slower), as in the token-mask mode and for key sequences under 8192.  (The gain depends on
     // the data: on i.i.d. normal inputs, where no quarter of a score tile is ever skipped and the softmax step is
     // longer, two issuers are level with one at 8192 keys and 1 % behind at 16384.)
     reg_dealloc<72>();
@@ -491,7 +492,7 @@ dense_attn_kernel(const __grid_constant__ CUtensorMap mq, const __grid_constant_
           continue;
         }
         float mx0, mx1;
-        // with rotating buffers the tile's previous P V product may still be running when its next scores are there
+        // with rotating scores the tile's previous P V product may still be running when its next scores are there
         auto quiet = [&]() {
           if (ROT) {
             if (!mbar_wait(bar(BAR_PV_DONE + t), (g - 1) & 1, ab, p.err, 303)) ok = false;

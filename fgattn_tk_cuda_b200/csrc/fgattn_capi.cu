@@ -588,9 +588,9 @@ int token_setup(fg::TokenParams& p, CUtensorMap& mq, CUtensorMap& mo, void* o, c
   return FGATTN_OK;
 }
 
-// The order of the thread blocks (len[item * subs + j], j < subs, of len_rows per unit: what item is long by) and the kernel.
+// The order of the thread blocks and the kernel.
 int token_launch(fg::TokenParams& p, const CUtensorMap& mq, const CUtensorMap& mo, int n_units, int D, int kv_rows,
-                 void* workspace, const int* len, int len_rows, int subs, int shift, cudaStream_t st) {
+                 void* workspace, cudaStream_t st) {
   int sms = 0;
   int r = sm_count(&sms);
   if (r) return r;
@@ -604,9 +604,11 @@ int token_launch(fg::TokenParams& p, const CUtensorMap& mq, const CUtensorMap& m
     group = std::max(1, std::min(group, n_units));
     const int n_groups = (n_units + group - 1) / group;
     group = (n_units + n_groups - 1) / n_groups;                      // groups of equal size
+    int shift = 0;
+    while ((p.mask_stride >> shift) >= 1024) ++shift;                   // bucketed list lengths
     int* ws = static_cast<int*>(workspace);
-    r = launch_behind(fg::sparse_order_kernel, dim3((n_units + group - 1) / group), 1024, 0, st, len, ws + 4, ws, len_rows, p.pairs,
-                      n_units, group, subs, 1, shift, nullptr);
+    r = launch_behind(fg::sparse_order_kernel, dim3((n_units + group - 1) / group), 1024, 0, st, p.kv_cnt, ws + 4, ws, p.nqb, p.pairs,
+                      n_units, group, 2, 1, shift, nullptr);
     if (r) return r;
     p.order = ws + 4;
   }
@@ -696,9 +698,7 @@ int fgattn_sp_attn(void* o, const void* q, const void* k, const void* v, const i
     if (r) return r;
     p.route = route;
   }
-  int shift = 0;
-  while ((mask_stride >> shift) >= 1024) ++shift;                     // bucketed list lengths
-  return token_launch(p, mq, mo, n_units, D, kv_rows, workspace, kv_num_indices, p.nqb, 2, shift, st);
+  return token_launch(p, mq, mo, n_units, D, kv_rows, workspace, st);
 }
 
 size_t fgattn_sp_attn_token_workspace_bytes(int batch, int heads, int seq, int kv_rows) {

@@ -24,7 +24,7 @@ __device__ __forceinline__ void online_init(OnlineState& st) {
 
 // Multiplies one row of the accumulator (D fp32 columns at o_addr) by alpha.  Nothing may still be adding to it.  Where
 // the query tile has one score buffer, the commit that published its scores covers its previous P*V product too.  With
-// rotating score buffers the scores come while that product may still be running: the caller waits for it first.
+// rotating scores they come while that product may still be running: the caller waits for it first.
 template <int D>
 __device__ __forceinline__ void rescale_accumulator(uint32_t o_addr, float alpha) {
 #pragma unroll
@@ -201,12 +201,10 @@ __device__ __forceinline__ void quarter_probs(uint32_t (&r)[32], float qmax, flo
 // against the offset as it stands, before the tile's maximum is known and while three quarters of the scores are still on
 // their way from tensor memory.  Where some row of the warp turns out to need a larger offset, nothing has been
 // written yet: that first quarter is loaded again and the probabilities of all quarters taken against the new one.  The
-// results are those of softmax_online_step bit for bit (backwards the row sums add up in another order).  Taken at D = 64, where the softmax bounds a step: (2, 16, 4096, 64),
-// i.i.d. normal q and k, 0.224 -> 0.217 ms.  With scores so far apart that the offset moves in most tiles (deviation of
-// q and k 2 / 3 / 6) softmax_online_step alone takes 0.232 / 0.239 / 0.241 ms, this with the rotating score buffers that
-// the dense kernel had then 0.225 / 0.239 / 0.247 (0.244 / 0.265 / 0.272 when a tile was done over from its maximum on).
-// At D = 128 it is level to 2.5 % slower (32768 x 512 keys 0.374 -> 0.384 ms): there the two products and the hand-offs
-// pace a step.
+// results are those of softmax_online_step bit for bit (backwards the row sums add up in another order).  Taken by the
+// dense kernel at D = 64, where the softmax bounds a step ((2, 16, 4096, 64), i.i.d. normal q and k, 0.224 -> 0.217 ms), and by
+// the full steps of the token lists, whose softmax is a link of a slot's chain, at both head dimensions.  The dense kernel at
+// D = 128 is level to 2.5 % slower with it (32768 x 512 keys 0.374 -> 0.384 ms): two products and their hand-offs pace a step.
 // `backwards` (warp-uniform): the quarters are taken last to first.  Only the first one taken is ever loaded again, so the
 // columns of the other half of the tile may be overwritten as soon as `loaded` has been called.
 template <int D, int POLY = 2, bool SKIP = true, class Quiet = NoWait, class Loaded = NoWait>
